@@ -3,6 +3,7 @@
 #include "../../include/care_b200.h"
 #include "hostio.hpp"
 #include "readfile.hpp"
+#include "align_tc.cuh"
 #include "kernels.cuh"
 #include "mlp.hpp"
 #include "parse.hpp"
@@ -923,6 +924,12 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
     // length classes of the alignment (not with mirror pairs, whose work list pairs equal lengths)
     const bool classes = tu.align_classes != 0 && tu.pair_mirror == 0;
     if (classes) CK(ctx->d_cls.ensure(64), "alloc");
+    // the tensor-core alignment, except for the statistics form and the
+    // mappings that ask for another scan
+    const bool tc = tc_applies(o.max_error_rate, o.min_overlap, o.min_overlap_ratio) && !ctx->count_words &&
+                    tu.align_warp == 0 && !classes;
+    const TcLayout tcl = tc_layout(ctx->max_len, ctx->opt.min_overlap, ctx->opt.min_overlap_ratio);
+    if (tc) CK(cudaFuncSetAttribute(k_align_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcl.total), "smem attr");
     const int qb = ctx->has_qual ? ctx->opt.quality_bits : 0;
     const size_t msmem = msa_smem_bytes(ctx->max_len, ctx->seq_pitch, ctx->has_qual ? ctx->qual_pitch : 0, qb, emit,
                                         32 * jb * warps);
@@ -933,8 +940,8 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
         CK(ctx->d_cand_anchor.ensure(cap * 4), "alloc candidates");
         CK(ctx->d_ares.ensure(cap * sizeof(AlignRes)), "alloc alignments");
         CK(ctx->d_recs.ensure(cap * sizeof(CandRec)), "alloc records");
-        if (tu.pair_order) CK(ctx->d_pair_order.ensure(cap * 4), "alloc pair order");
-        if (tu.pair_mirror) CK(ctx->d_pair_work.ensure(cap * 8), "alloc mirror work list");
+        if (tu.pair_order && !tc) CK(ctx->d_pair_order.ensure(cap * 4), "alloc pair order");
+        if (tu.pair_mirror) CK(ctx->d_pair_work.ensure(cap * (tc ? 4 : 8)), "alloc mirror work list");
         if (classes) CK(ctx->d_pair_class.ensure(cap * 4), "alloc pair classes");
         const unsigned long long ccap = ctx->corr_cap;
         CK(ctx->d_cid.ensure(ccap * 4), "alloc");
@@ -1024,14 +1031,34 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
                 ++launches;
             }
             EQ(mark(1), "event");
-            if (tu.pair_order) {
+            if (tc) {
+                if (tu.pair_mirror) {
+                    k_mirror_index<<<(unsigned)((cap + 255) / 256), 256, 0, st>>>(
+                        r, first, count, ctx->d_cand_ids.as<uint32_t>(), ctx->d_cand_anchor.as<uint32_t>(),
+                        ctx->d_seg_off.as<uint32_t>(), ctx->d_seg_cnt.as<uint32_t>(), counters, cap, status,
+                        ctx->d_pair_work.as<uint32_t>());
+                    EQ(cudaGetLastError(), "k_mirror_index");
+                    ++launches;
+                }
+                const unsigned resident = (unsigned)(ctx->sms * tc_ctas(tcl));
+                const uint32_t splits = tc_splits(count, resident);
+                const unsigned g = (unsigned)std::min<uint64_t>((uint64_t)count * splits, resident);
+                k_align_tc<<<g, kTcBlock, tcl.total, st>>>(
+                    o, r, first, count, ctx->d_cand_ids.as<uint32_t>(), ctx->d_seg_off.as<uint32_t>(),
+                    ctx->d_seg_cnt.as<uint32_t>(), counters, cap, status, ctx->d_ares.as<AlignRes>(), counters + 3,
+                    tu.pair_mirror ? ctx->d_pair_work.as<uint32_t>() : nullptr,
+                    reinterpret_cast<unsigned int*>(counters + 11), splits, tcl);
+                EQ(cudaGetLastError(), "k_align_tc");
+                ++launches;
+            }
+            if (tu.pair_order && !tc) {
                 k_pair_order<<<count, 128, 0, st>>>(r, ctx->d_cand_ids.as<uint32_t>(), ctx->d_seg_off.as<uint32_t>(),
                                                     ctx->d_seg_cnt.as<uint32_t>(), count, status,
                                                     ctx->d_pair_order.as<uint32_t>());
                 EQ(cudaGetLastError(), "k_pair_order");
                 ++launches;
             }
-            if (tu.pair_mirror) {
+            if (tu.pair_mirror && !tc) {
                 k_pair_mirror<256><<<(unsigned)((cap + 255) / 256), 256, 0, st>>>(
                     r, first, count, ctx->d_cand_ids.as<uint32_t>(), ctx->d_cand_anchor.as<uint32_t>(),
                     ctx->d_seg_off.as<uint32_t>(), ctx->d_seg_cnt.as<uint32_t>(), counters, cap, status,
@@ -1064,7 +1091,7 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
                     EQ(align_dispatch(tu.align_block, align_class_width(c), ac, st), "k_align");
                     ++launches;
                 }
-            } else {
+            } else if (!tc) {
                 EQ(align_dispatch(tu.align_block, nw, aa, st), "k_align");
                 ++launches;
             }
@@ -1138,6 +1165,7 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
         const unsigned long long rb_elems = ctx->h_small.as<unsigned long long>()[9];
         const unsigned long long rb_anchors = ctx->h_small.as<unsigned long long>()[10];
         const int stw = *(int*)(ctx->h_small.as<char>() + 88);
+        if (stw & kStatusTensorWait) return fail(ctx, CARE_B200_ECUDA, "tensor-core completion wait ran out");
         if (stw & kStatusColumns) return fail(ctx, CARE_B200_ELIMIT, "MSA wider than the kernel's column capacity");
         bool again = false;
         if ((stw & kStatusCandOverflow) || used > cap) {

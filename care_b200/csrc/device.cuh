@@ -159,6 +159,7 @@ enum : int {
     kStatusCorrOverflow = 2,          // candidate-correction arena too small
     kStatusColumns = 4,               // more MSA columns than the kernel holds
     kStatusFeatOverflow = 8,          // decision-column arena too small
+    kStatusTensorWait = 16,           // a tensor-core completion wait ran out
 };
 
 // MurmurHash3 64-bit finalizer (the published fmix64), as used by the
@@ -492,21 +493,18 @@ CB_HD ShdResult shifted_hamming(const uint32_t (&Ah)[NW + 2], const uint32_t (&A
 CB_HD int choose_orientation(const ShdResult& f, const ShdResult& r, int La,
                                                   float min_overlap_ratio, int min_overlap,
                                                   float maxErrorRate) {
-    int ret = 3;
     const int lo = f2i_rz(fmul_rn((float)La, min_overlap_ratio));
     const int mo = lo > min_overlap ? lo : min_overlap;
-    if (f.valid && f.overlap >= mo) {
-        if (r.valid && r.overlap >= mo) {
-            const float ratio = fdiv_rn((float)f.nops, (float)f.overlap);
-            const float rratio = fdiv_rn((float)r.nops, (float)r.overlap);
-            if (ratio < rratio) { if (ratio < maxErrorRate) ret = 1; }
-            else if (rratio < ratio) { if (rratio < maxErrorRate) ret = 2; }
-            else if (ratio < maxErrorRate) ret = f.overlap > r.overlap ? 1 : 2;
-        } else if (fdiv_rn((float)f.nops, (float)f.overlap) < maxErrorRate) ret = 1;
-    } else if (r.valid && r.overlap >= mo) {
-        if (fdiv_rn((float)r.nops, (float)r.overlap) < maxErrorRate) ret = 2;
-    }
-    return ret;
+    const bool fo = f.valid && f.overlap >= mo, ro = r.valid && r.overlap >= mo;
+    // one division per orientation, outside the branches (a warp's lanes take
+    // all of them); an orientation that does not count never wins
+    const float big = 3.402823466e+38f;
+    const float ratio = fo ? fdiv_rn((float)f.nops, (float)f.overlap) : big;
+    const float rratio = ro ? fdiv_rn((float)r.nops, (float)r.overlap) : big;
+    if (!fo && !ro) return 3;
+    if (fo && ro && ratio == rratio) return ratio < maxErrorRate ? (f.overlap > r.overlap ? 1 : 2) : 3;
+    if (ratio < rratio) return ratio < maxErrorRate ? 1 : 3;
+    return rratio < maxErrorRate ? 2 : 3;
 }
 
 // feq / fleq / fgeq (include/hostdevicefunctions.cuh:9-29).

@@ -9,6 +9,7 @@
 // in one file-scope device array of fixed size, kNoAllocScratchBytes.
 #include "../../include/care_b200.h"
 #include "hostio.hpp"
+#include "align_tc.cuh"
 #include "kernels.cuh"
 
 #include <algorithm>
@@ -25,6 +26,7 @@ constexpr unsigned long long kNoAllocMaxPairs = CARE_B200_NOALLOC_MAX_PAIRS;
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kOffCounters = 0;                                          // u64[8]
 constexpr size_t kOffStatus = 64;                                           // int[4]
+constexpr size_t kOffCursor = 128;                                          // u32: next anchor of the alignment
 constexpr size_t kOffSegOff = 256;
 constexpr size_t kOffSegCnt = align256(kOffSegOff + 4ull * kNoAllocMaxAnchors);
 constexpr size_t kOffCandIds = align256(kOffSegCnt + 4ull * kNoAllocMaxAnchors);
@@ -182,23 +184,38 @@ extern "C" int care_b200_correct_range_noalloc(const care_b200_options* opt, con
         o, r, static_cast<const TableDesc*>(tables->descs), static_cast<const Slot*>(tables->slots), tables->values,
         nullptr, first_anchor, num_anchors, set_log2, nullptr, nullptr, cand_ids, cand_anchor, seg_off, seg_cnt, counters, kNoAllocMaxPairs,
         dstatus);
-    // the pairs the candidate pass found size the alignment grid; a count
-    // above the array's pair capacity ends the call here
-    unsigned long long npairs = 0;
-    if (cudaMemcpyAsync(&npairs, counters, sizeof(npairs), cudaMemcpyDeviceToHost, st) != cudaSuccess)
-        return CARE_B200_ECUDA;
-    if (cudaStreamSynchronize(st) != cudaSuccess) return CARE_B200_ECUDA;
-    if (npairs > kNoAllocMaxPairs) return CARE_B200_ELIMIT;
-    const unsigned ablocks = (unsigned)std::max<unsigned long long>((npairs + 127) / 128, 1);
-    const int nw = (r.max_len + 31) / 32;
+    if (tc_applies(o.max_error_rate, o.min_overlap, o.min_overlap_ratio)) {
+        // the grid follows the anchors; a pair count above the array's
+        // capacity is in the status word, which every later kernel looks at
+        const TcLayout tcl = tc_layout(r.max_len, o.min_overlap, o.min_overlap_ratio);
+        int sms = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return CARE_B200_ECUDA;
+        if (cudaFuncSetAttribute(k_align_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcl.total) != cudaSuccess)
+            return CARE_B200_ECUDA;
+        const unsigned resident = (unsigned)(sms * tc_ctas(tcl));
+        const uint32_t splits = tc_splits(num_anchors, resident);
+        k_align_tc<<<std::min<unsigned>(num_anchors * splits, resident), kTcBlock, tcl.total, st>>>(
+            o, r, first_anchor, num_anchors, cand_ids, seg_off, seg_cnt, counters, kNoAllocMaxPairs, dstatus, ares,
+            nullptr, nullptr, reinterpret_cast<unsigned int*>(scratch + kOffCursor), splits, tcl);
+    } else {
+        // the pairs the candidate pass found size the alignment grid; a count
+        // above the array's pair capacity ends the call here
+        unsigned long long npairs = 0;
+        if (cudaMemcpyAsync(&npairs, counters, sizeof(npairs), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+            return CARE_B200_ECUDA;
+        if (cudaStreamSynchronize(st) != cudaSuccess) return CARE_B200_ECUDA;
+        if (npairs > kNoAllocMaxPairs) return CARE_B200_ELIMIT;
+        const unsigned ablocks = (unsigned)std::max<unsigned long long>((npairs + 127) / 128, 1);
+        const int nw = (r.max_len + 31) / 32;
 #define LAUNCH_ALIGN(NW)                                                                                    \
-    k_align<128, NW><<<ablocks, 128, 0, st>>>(o, r, first_anchor, cand_ids, cand_anchor, seg_off, seg_cnt,  \
-                                              counters, kNoAllocMaxPairs, dstatus, ares, nullptr, nullptr, nullptr, nullptr, nullptr)
-    if (nw <= 4) LAUNCH_ALIGN(4);
-    else if (nw <= 5) LAUNCH_ALIGN(5);
-    else if (nw <= 6) LAUNCH_ALIGN(6);
-    else LAUNCH_ALIGN(8);
+        k_align<128, NW><<<ablocks, 128, 0, st>>>(o, r, first_anchor, cand_ids, cand_anchor, seg_off, seg_cnt,  \
+                                                  counters, kNoAllocMaxPairs, dstatus, ares, nullptr, nullptr, nullptr, nullptr, nullptr)
+        if (nw <= 4) LAUNCH_ALIGN(4);
+        else if (nw <= 5) LAUNCH_ALIGN(5);
+        else if (nw <= 6) LAUNCH_ALIGN(6);
+        else LAUNCH_ALIGN(8);
 #undef LAUNCH_ALIGN
+    }
     MsaOut mo{};
     mo.status = status;
     mo.nedits = num_edits;
@@ -234,6 +251,7 @@ extern "C" int care_b200_correct_range_noalloc(const care_b200_options* opt, con
     int hstatus = 0;
     if (cudaMemcpyAsync(&hstatus, dstatus, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return CARE_B200_ECUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return CARE_B200_ECUDA;
+    if (hstatus & kStatusTensorWait) return CARE_B200_ECUDA;
     if (hstatus & (kStatusCandOverflow | kStatusColumns)) return CARE_B200_ELIMIT;
     return CARE_B200_OK;
 }

@@ -1,0 +1,125 @@
+// Host emulation of the tensor-core alignment (care_b200/csrc/align_tc.cuh)
+// for one anchor and its candidates: the operand images and the addresses the
+// matrix descriptors form, the sums, both threshold forms, the exact counts
+// and the keys. Test infrastructure only.
+#include "../../care_b200/csrc/tc_math.cuh"
+
+#include <cstring>
+#include <vector>
+
+using namespace careb200;
+
+static float e4m3(uint8_t b) { return b == 0x38 ? 1.0f : b == 0xB8 ? -1.0f : b == 0 ? 0.0f : 1e30f; }
+
+// rows: n candidates of `pitch` words. out: 16 ints per candidate -- score,
+// overlap, shift, nops, valid of (A, C), of (A, rc C) and of (C, A), then the
+// orientation. per_column: the threshold form of mixed lengths. Returns the
+// possible shifts listed, -1 on a byte no operand holds, -2 on an index past
+// a buffer.
+extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch, const int* len, int n, int max_len,
+                     int min_overlap, float rate, float ratio, float est, int per_column, int* out) {
+    const TcLayout lay = tc_layout(max_len, min_overlap, ratio);
+    const int W = lay.W, RS = lay.RS, XL = lay.XL;
+    if (n > kTcMaxItems) return -2;
+    const int lo = f2i_rz(fmul_rn((float)La, ratio));
+    const int minov = min_overlap > lo ? min_overlap : lo;
+    const int smax = La - minov, nwa = (La + 15) / 16, nI = (n + 7) & ~7;
+    int maxl = 0;
+    for (int i = 0; i < n; ++i) maxl = len[i] > maxl ? len[i] : maxl;
+    const int smin = minov - maxl;
+    const int ntiles = (smax < 0 || maxl < minov) ? 0 : (smax - smin + 128) >> 7;
+    if (ntiles > lay.tiles) return -2;
+    std::vector<uint32_t> aw(kMaxLen / 16 + 2, 0u), fwp((size_t)kTcMaxItems * RS + 1, 0x5a5a5a5au), rw((size_t)kTcMaxItems * RS, 0u);
+    uint32_t* fw = fwp.data() + 1;                     // a word before the first row is read
+    for (int i = 0; i < nwa; ++i) aw[i] = a[i];
+    std::vector<uint8_t> top(lay.b - lay.top), b((size_t)2 * kTcMaxItems * 16 * W, 0x7f);
+    for (int i = 0; i < n; ++i)
+        for (int w = 0; w < W; ++w) fw[i * RS + w] = 16 * w < len[i] ? rows[(size_t)i * pitch + w] : 0u;
+    for (int i = 0; i < n; ++i)
+        for (int c = 0; c < W; ++c)
+            for (int rev = 0; rev < 2; ++rev) {
+                uint32_t x = fw[i * RS + c];
+                if (rev) rw[i * RS + c] = x = tc_rc_word(&fw[i * RS], len[i], c);
+                uint32_t w[4];
+                tc_expand(x, w);
+                if (len[i] - 16 * c < 16) tc_mask(w, 0, len[i] - 16 * c);
+                const int row = rev * nI + i;
+                std::memcpy(&b[(size_t)(row >> 3) * (128 * W) + c * 128 + (row & 7) * 16], w, 16);
+            }
+    std::vector<uint32_t> q((size_t)(XL + 1) * 4);
+    if ((uint32_t)q.size() * 4 > lay.top - lay.q) return -2;
+    for (int x = 0; x <= XL; ++x) {
+        uint32_t w[4];
+        tc_q_chunk(aw.data(), nwa, La, smax - 127 - 128 * (lay.tiles - 1) + 16 * x, w);
+        std::memcpy(&q[4 * x], w, 16);
+    }
+    for (int rho = 0; rho < 16; ++rho)
+        for (int x = 0; x < XL; ++x) {
+            uint32_t e[5], w[4];
+            std::memcpy(e, &q[4 * x + (rho >> 2)], 20);
+            tc_shift16(e, rho & 3, w);
+            if ((size_t)(rho * XL + x) * 16 + 16 > top.size()) return -2;
+            std::memcpy(&top[(size_t)(rho * XL + x) * 16], w, 16);
+        }
+    for (int idx = 0; idx < kTcMaxItems * W; ++idx)
+        if ((int)(((uint32_t)idx * lay.magic_w) >> 16) != idx / W) return -2;
+    std::vector<uint32_t> key((size_t)3 * n, 0xFFFFFFFFu);
+    const float kappa = 1.0f - 2.0f * rate;
+    int hits = 0;
+    const int K = 32 * ((maxl + 31) / 32);
+    for (int t = 0; t < ntiles; ++t)
+        for (int m = 0; m < 128; ++m) {
+            const int s = smax - 127 - 128 * t + tc_row_shift(m);
+            for (int col = 0; col < 2 * n; ++col) {
+                const int rev = col >= n, it = col - rev * n, row = rev * nI + it, Lc = len[it];
+                float d = 0.0f;
+                for (int k = 0; k < K; ++k) {
+                    const size_t ea = (size_t)8 * (lay.tiles - 1 - t) * 16 + (size_t)(m >> 3) * (16 * XL) + (k >> 4) * 16 + (m & 7) * 16 + (k & 15);
+                    const size_t eb = (size_t)(row >> 3) * (128 * W) + (k >> 4) * 128 + (row & 7) * 16 + (k & 15);
+                    if (ea >= top.size() || eb >= b.size()) return -2;
+                    d += e4m3(top[ea]) * e4m3(b[eb]);
+                }
+                if (d > 1e6f || d < -1e6f) return -1;
+                if (s < smin) continue;
+                float thr = 1e9f;
+                if (!per_column) {
+                    const int ov = tc_overlap(s, La, Lc);
+                    if (ov >= minov) thr = tc_threshold(ov, f2i_rz(fmul_rn((float)ov, rate)));
+                } else {
+                    const int u = s > 0 ? s : 0;
+                    const float c1 = kappa * (float)(La - u) + kTcSlack, c2 = kappa * (float)(s - u) + kTcSlack;
+                    const float cm = kappa * (float)minov + kTcSlack;
+                    const float e = kappa * (float)Lc + c2;
+                    thr = e < c1 ? e : c1;
+                    thr = thr > cm ? thr : cm;
+                }
+                if (!(d >= thr)) continue;
+                ++hits;
+                const int ov = tc_overlap(s, La, Lc);
+                if (ov < minov) continue;
+                const uint32_t* cr = rev ? &rw[it * RS] : &fw[it * RS];
+                const int mex = f2i_rz(fmul_rn((float)ov, rate));
+                int mm = 0;
+                for (int part = 0; part < 4; ++part)
+                    mm += s >= 0 ? tc_mismatches(aw.data(), cr, s, ov, part, 4) : tc_mismatches(cr, aw.data(), -s, ov, part, 4);
+                if (mm >= mex) continue;
+                const uint32_t sc = (uint32_t)(mm + La + Lc - 2 * ov) << 10;
+                uint32_t& ka = key[rev * n + it];
+                ka = ka < (sc | tc_rank(s)) ? ka : sc | tc_rank(s);
+                uint32_t& kc = key[2 * n + it];
+                if (!rev) kc = kc < (sc | tc_rank(-s)) ? kc : sc | tc_rank(-s);
+            }
+        }
+    for (int it = 0; it < n; ++it) {
+        const ShdResult f = tc_result(key[it], La, len[it]), r = tc_result(key[n + it], La, len[it]),
+                        g = tc_result(key[2 * n + it], len[it], La);
+        const ShdResult* rs[3] = {&f, &r, &g};
+        int* o = out + 16 * it;
+        for (int k = 0; k < 3; ++k) {
+            o[5 * k] = rs[k]->score; o[5 * k + 1] = rs[k]->overlap; o[5 * k + 2] = rs[k]->shift;
+            o[5 * k + 3] = rs[k]->nops; o[5 * k + 4] = rs[k]->valid;
+        }
+        o[15] = choose_orientation(f, r, La, ratio, min_overlap, fmul_rn(est, 4.0f));
+    }
+    return hits;
+}
