@@ -576,7 +576,7 @@ def main():
                                  "peak": ip["msa_elements_per_s"] if ip else None,
                                  "frac": (stats["msa_elements"] / (stage[2] / 1e3) / ip["msa_elements_per_s"])
                                  if ip else None,
-                                 "work": "bases added to column sums (anchor and candidates, every build), "
+                                 "work": "bases of the MSAs' rows (anchor and candidates, every build), "
                                          "counted by k_msa",
                                  "work_per_step": stats["msa_elements"],
                                  "rebuild_elements_per_step": stats["msa_rebuild_elements"],

@@ -816,7 +816,7 @@ struct MsaArgs {
     const uint32_t* cand_ids; const uint32_t* seg_off; const uint32_t* seg_cnt; const AlignRes* ares;
     CandRec* recs; MsaOut out; int* status; size_t smem;
     bool queue; int sms; int grid;             // grid: resident CTAs of the queue form (prepare)
-    int jb;                                    // 32-column blocks per warp
+    MsaGrid mgrid;                             // the staged rows' grid
 };
 
 // prepare (host only: attributes, occupancy) or launch one MSA variant
@@ -832,11 +832,11 @@ cudaError_t msa_go(MsaArgs& a, bool prepare, cudaStream_t st) {
         return e;
     }
     if (a.queue)
-        k_msa_queue<B, QB, E><<<a.grid, B, a.smem, st>>>(a.o, a.r, a.first, a.count, a.jb, a.order, a.cursor,
+        k_msa_queue<B, QB, E><<<a.grid, B, a.smem, st>>>(a.o, a.r, a.first, a.count, a.mgrid, a.order, a.cursor,
                                                         a.cand_ids, a.seg_off, a.seg_cnt, a.ares, a.recs, a.out,
                                                         a.status);
     else
-        k_msa<B, QB, E><<<a.count, B, a.smem, st>>>(a.o, a.r, a.first, a.count, a.jb, a.order, a.cand_ids,
+        k_msa<B, QB, E><<<a.count, B, a.smem, st>>>(a.o, a.r, a.first, a.count, a.mgrid, a.order, a.cand_ids,
                                                     a.seg_off, a.seg_cnt, a.ares, a.recs, a.out, a.status);
     return cudaGetLastError();
 }
@@ -911,15 +911,7 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
         CK(ctx->d_touched.ensure(count), "alloc");
         CK(ctx->d_mlp_err.ensure(16), "alloc");
     }
-    // widest possible MSA: La + 2*Lmax - 2*minoverlap(La), maximised over La
-    int maxcols = 1;
-    for (int la = 1; la <= ctx->max_len; ++la) {
-        const int lo = (int)((float)la * ctx->opt.min_overlap_ratio);
-        const int mo = std::max(ctx->opt.min_overlap, lo);
-        maxcols = std::max(maxcols, la + 2 * ctx->max_len - 2 * std::min(mo, ctx->max_len));
-    }
     const int warps = tu.msa_warps == 8 ? 8 : 4;
-    const int jb = (maxcols + 32 * warps - 1) / (32 * warps);
     const int nw = (ctx->max_len + 31) / 32;           // bit-plane width: 32-base words of the longest read
     // length classes of the alignment (not with mirror pairs, whose work list pairs equal lengths)
     const bool classes = tu.align_classes != 0 && tu.pair_mirror == 0;
@@ -931,8 +923,8 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
     const TcLayout tcl = tc_layout(ctx->max_len, ctx->opt.min_overlap, ctx->opt.min_overlap_ratio);
     if (tc) CK(cudaFuncSetAttribute(k_align_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcl.total), "smem attr");
     const int qb = ctx->has_qual ? ctx->opt.quality_bits : 0;
-    const size_t msmem = msa_smem_bytes(ctx->max_len, ctx->seq_pitch, ctx->has_qual ? ctx->qual_pitch : 0, qb, emit,
-                                        32 * jb * warps);
+    const MsaGrid mgrid = msa_grid(ctx->max_len, qb, o.correct_candidates, o.new_columns);
+    const size_t msmem = msa_smem_bytes(mgrid, ctx->max_len, emit);
 
     for (int attempt = 0; attempt < 8; ++attempt) {
         const unsigned long long cap = ctx->cand_cap;
@@ -988,7 +980,7 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
         MsaArgs ma{o, r, first, count, tu.msa_order ? ctx->d_order.as<uint32_t>() : nullptr,
                    reinterpret_cast<unsigned int*>(counters + 4), ctx->d_cand_ids.as<uint32_t>(),
                    ctx->d_seg_off.as<uint32_t>(), ctx->d_seg_cnt.as<uint32_t>(), ctx->d_ares.as<AlignRes>(),
-                   ctx->d_recs.as<CandRec>(), mo, status, msmem, tu.msa_queue != 0, ctx->sms, 0, jb};
+                   ctx->d_recs.as<CandRec>(), mo, status, msmem, tu.msa_queue != 0, ctx->sms, 0, mgrid};
         CK(msa_dispatch(warps, qb, emit, ma, true, ctx->stream), "MSA launch setup");
 
         cudaStream_t st = ctx->stream;
@@ -1166,7 +1158,6 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
         const unsigned long long rb_anchors = ctx->h_small.as<unsigned long long>()[10];
         const int stw = *(int*)(ctx->h_small.as<char>() + 88);
         if (stw & kStatusTensorWait) return fail(ctx, CARE_B200_ECUDA, "tensor-core completion wait ran out");
-        if (stw & kStatusColumns) return fail(ctx, CARE_B200_ELIMIT, "MSA wider than the kernel's column capacity");
         bool again = false;
         if ((stw & kStatusCandOverflow) || used > cap) {
             // pair indices and segment offsets are 32-bit

@@ -157,7 +157,6 @@ enum : int {
     kStatusOk = 0,
     kStatusCandOverflow = 1,          // candidate arena too small, rerun with more space
     kStatusCorrOverflow = 2,          // candidate-correction arena too small
-    kStatusColumns = 4,               // more MSA columns than the kernel holds
     kStatusFeatOverflow = 8,          // decision-column arena too small
     kStatusTensorWait = 16,           // a tensor-core completion wait ran out
 };

@@ -725,15 +725,27 @@ k_align_warp(DevOptions o, DevReads r, uint32_t first, const uint32_t* __restric
 //   getCorrectedCandidates            src/msa.cpp:457-522
 //   makeOutputOfTask (edits)          include/corrector.hpp:1639-1761
 //
-// Layout: warp w owns the 32-column blocks w, w+NWARP, ...; lane l owns
-// column 32*block + l. A column's sums are accumulated by its owner, anchor
-// first and then candidates in list order, with separate IEEE multiply and
-// add (no FMA) -- the reference's order and rounding, so the sums are
-// bit-identical. A warp skips a candidate that covers none of a block's
-// columns (a warp-uniform test). Candidate rows are staged in shared memory
-// as their packed sequence and quality words (all warps loading, eight rows
-// in flight per lane) and read in place; they stay staged across refinement
-// rebuilds when the candidate list fits (up to 128 rows in 16 KB).
+// What the anchor's result needs of the MSA: per anchor column the consensus,
+// its support and the counts. A column whose rows all hold the anchor's base
+// has that base as consensus with support exactly 1 (one of the four sums is
+// non-zero, and it is the column weight), whatever its sums are. So the rows
+// are compared with the anchor 16 bases at a time while they are staged, and
+// only the columns where some row differs (disputed columns, a quarter of
+// them at 30x) get sums: one lane per column, its rows in list order, anchor
+// first, with separate IEEE multiply and add (no FMA) -- the reference's order
+// and rounding, so the sums are bit-identical. Coverage comes from the rows'
+// ends. Columns outside the anchor are summed only for candidate correction,
+// within its new_columns of the anchor.
+//
+// Rows are staged in shared memory as the words of the anchor's own 16-base
+// grid (word g holds anchor positions 16 g .. 16 g + 15, turned into the
+// aligned orientation), a thread per (row, word); the anchor is row 0. They
+// stay staged across refinement rebuilds when the candidate list fits (up to
+// 128 rows in 16 KB).
+// Bound: instruction issue. Measured against sums of every column with the
+// rows staged whole: 1M 150 bp paired-end reads at 30x 13.0 ms (20.7), 400k
+// reads of 50-250 bases 8.8 ms (18.2), 1.3M reads at 50x 22.4 ms (38.4), 128
+// anchors 0.17 ms (0.45).
 // ---------------------------------------------------------------------------
 struct MsaOut {
     uint8_t* status;
@@ -752,10 +764,11 @@ struct MsaOut {
     uint32_t* feat_meta;
     unsigned long long* feat_count;
     unsigned long long feat_cap;
-    // elements added to column sums (anchor and candidate bases, every
-    // build): the MSA stage's roofline work; may be null
+    // bases of the MSAs' rows (anchor and candidates, every build): the MSA
+    // stage's roofline work (the sums of undisputed columns are not formed);
+    // may be null
     unsigned long long* elem_count;
-    // refinement statistics, may be null: [0] elements added by rebuilds
+    // refinement statistics, may be null: [0] the rows' bases in rebuilds
     // (builds after the first), [1] anchors rebuilt at least once
     unsigned long long* rebuild_count;
 };
@@ -764,77 +777,59 @@ constexpr int kNumFeatures = 24;
 
 constexpr int kStageMax = 128;        // candidate rows held in shared memory, at most
 constexpr int kStageBudget = 16384;   // bytes of staged rows
-constexpr int kStageGuard = 32;       // bytes before and after the staged rows
 
-// words of a staged row (qb: the quality encoding the sums read). The bases
-// are realigned to the anchor's 16-base grid, so they take one word more than
-// the read's pitch; 1- and 8-bit quality codes follow on their own grids (32
-// and 4 codes per word), 2-bit codes are interleaved with the bases as word
-// pairs {bases, qualities} of the same 16 positions.
-__host__ __device__ inline int msa_slot_words(int seq_pitch, int qual_pitch, int qb) {
-    if (qb == 0) return seq_pitch + 1;
-    if (qb == 2) return 2 * ((seq_pitch > qual_pitch ? seq_pitch : qual_pitch) + 1);
-    return seq_pitch + 1 + qual_pitch + 1;
+// The staged rows' grid: `words` 16-base words, `edge` of them on each side of
+// the anchor (columns outside it that candidate correction reads), `wpg`
+// 32-bit words per grid word: the bases, then the qualities of the same
+// positions (16 1-bit codes in the high half, 16 2-bit codes, or 16
+// characters); per-column arrays hold 16 * words entries.
+struct MsaGrid {
+    int edge, words, wpg, rw, rows;
+    uint32_t magic;                   // x / words as the high word of x * magic (words > 1)
+};
+__host__ __device__ inline MsaGrid msa_grid(int max_len, int qb, int correct_candidates, int new_columns) {
+    MsaGrid g{};
+    const int nc = new_columns < 0 ? 0 : new_columns > kMaxLen ? kMaxLen : new_columns;
+    g.edge = correct_candidates ? (nc + 15) / 16 : 0;
+    g.words = (max_len + 15) / 16 + 2 * g.edge;
+    g.wpg = qb == 0 ? 1 : qb == 8 ? 5 : 2;
+    g.rw = g.words * g.wpg;
+    const int rows = kStageBudget / (g.rw * 4);
+    g.rows = rows > kStageMax ? kStageMax : (rows < 16 ? 16 : rows);
+    g.magic = (uint32_t)((0x100000000ull + (uint32_t)g.words - 1) / (uint32_t)g.words);
+    return g;
 }
 
-// candidate rows staged at once
-__host__ __device__ inline int msa_stage_rows(int seq_pitch, int qual_pitch, int qb) {
-    const int rows = kStageBudget / (msa_slot_words(seq_pitch, qual_pitch, qb) * 4);
-    return rows > kStageMax ? kStageMax : (rows < 16 ? 16 : rows);
-}
-
-// dynamic shared memory of k_msa: the anchor's decoded row, the staged
-// candidate rows (between two guard bands: a lane whose column lies outside
-// a row may read a few words past either end of it, and adds nothing); with
-// decision rows also three per-anchor-column weights; then the per-column
-// arrays of `maxcols` columns (four 16-bit counts, support, coverage,
-// consensus). Every part starts on a 16-byte boundary (maxcols is a multiple
-// of 128).
+// dynamic shared memory of k_msa: the staged rows (the anchor and `rows`
+// candidates), per anchor position the support and the four counts, with
+// decision rows three column weights, then the coverage, the column list and
+// the bases of the grid's columns. Every part starts on a 16-byte boundary.
 __host__ __device__ inline size_t msa_round16(size_t x) { return (x + 15) & ~(size_t)15; }
-__host__ __device__ inline size_t msa_raw_bytes(int seq_pitch, int qual_pitch, int qb) {
-    return msa_round16(2 * kStageGuard + (size_t)msa_stage_rows(seq_pitch, qual_pitch, qb) *
-                                             msa_slot_words(seq_pitch, qual_pitch, qb) * 4);
-}
-__host__ __device__ inline size_t msa_smem_bytes(int max_len, int seq_pitch, int qual_pitch, int qb, bool emit,
-                                                 int maxcols) {
-    const size_t elem = msa_round16((size_t)max_len * 2);
-    const size_t fw = emit ? msa_round16((size_t)3 * max_len * 4) : 0;
-    return elem + msa_raw_bytes(seq_pitch, qual_pitch, qb) + fw + (size_t)maxcols * (8 + 4 + 2 + 1);
+__host__ __device__ inline size_t msa_smem_bytes(const MsaGrid& g, int max_len, bool emit) {
+    const size_t cols = 16 * (size_t)g.words;
+    return msa_round16((size_t)(g.rows + 1) * g.rw * 4) + msa_round16((size_t)max_len * 4) + (size_t)max_len * 8 +
+           8 * (size_t)(max_len & 1) + (emit ? msa_round16((size_t)3 * max_len * 4) : 0) +
+           msa_round16((size_t)max_len * 2) + msa_round16(cols * 2) + cols;
 }
 
-// Realigned and reversed rows: a window of one word of codes whose first
-// code is code s0 of a source row (codes before the row and past its end
-// read as zero), the source row's words held one per lane in m (zero from
-// the row's pitch on; lane 31 zero for the 2- and 1-bit forms, whose pitches
-// are at most 16 and 8 words). Branch free: the row is read as if preceded
-// by one zero word, and a funnel shift with a zero count returns its high
-// word.
-// 2-bit codes, 16 per word, MSB first
-__device__ __forceinline__ uint32_t window2(uint32_t m, int s0) {
-    const int sc = max(s0 + 16, 0);
-    const int wi = sc >> 4;
-    const uint32_t a = __shfl_sync(0xffffffffu, m, (wi + 31) & 31);    // source word wi - 1
-    const uint32_t b = __shfl_sync(0xffffffffu, m, wi & 31);
-    return __funnelshift_l(b, a, 2 * (sc & 15));
+// The 16 2-bit codes from code b on of a packed row of n words; codes outside
+// the row are arbitrary.
+__device__ __forceinline__ uint32_t window2(const uint32_t* __restrict__ row, int n, int b) {
+    const int wi = b >> 4;
+    const uint32_t hi = __ldg(row + min(max(wi, 0), n - 1)), lo = __ldg(row + min(max(wi + 1, 0), n - 1));
+    return __funnelshift_l(lo, hi, 2 * (b & 15));
 }
-// 1-bit codes, 32 per word, MSB first
-__device__ __forceinline__ uint32_t window1(uint32_t m, int s0) {
-    const int sc = max(s0 + 32, 0);
-    const int wi = sc >> 5;
-    const uint32_t a = __shfl_sync(0xffffffffu, m, (wi + 31) & 31);
-    const uint32_t b = __shfl_sync(0xffffffffu, m, wi & 31);
-    return __funnelshift_l(b, a, sc & 31);
+// 1-bit codes, 32 per word, MSB first: 16 codes in the high half
+__device__ __forceinline__ uint32_t window1(const uint32_t* __restrict__ row, int n, int b) {
+    const int wi = b >> 5;
+    const uint32_t hi = __ldg(row + min(max(wi, 0), n - 1)), lo = __ldg(row + min(max(wi + 1, 0), n - 1));
+    return __funnelshift_l(lo, hi, b & 31);
 }
-// 8-bit codes, 4 per word, little-endian; source words 0..31 in m0, 32..63 in m1
-__device__ __forceinline__ uint32_t window8(uint32_t m0, uint32_t m1, int s0) {
-    const int sc = max(s0 + 4, 0);
-    const int wi = sc >> 2;
-    const int ia = wi - 1, ib = wi;
-    const uint32_t a0 = __shfl_sync(0xffffffffu, m0, ia & 31), a1 = __shfl_sync(0xffffffffu, m1, ia & 31);
-    const uint32_t b0 = __shfl_sync(0xffffffffu, m0, ib & 31), b1 = __shfl_sync(0xffffffffu, m1, ib & 31);
-    const uint32_t a = ia < 0 ? 0u : ia < 32 ? a0 : a1;
-    const uint32_t b = ib < 32 ? b0 : b1;
-    return __funnelshift_r(a, b, 8 * (sc & 3));
+// 4 characters from character b on, little-endian
+__device__ __forceinline__ uint32_t window8(const uint32_t* __restrict__ row, int n, int b) {
+    const int wi = b >> 2;
+    const uint32_t lo = __ldg(row + min(max(wi, 0), n - 1)), hi = __ldg(row + min(max(wi + 1, 0), n - 1));
+    return __funnelshift_r(lo, hi, 8 * (b & 3));
 }
 // reverse the 16 2-bit codes of a word, keeping each code's bits
 __device__ __forceinline__ uint32_t rev2(uint32_t w) {
@@ -872,116 +867,91 @@ __device__ __forceinline__ void msa_add8(float& wA, float& wC, float& wG, float&
 // The whole MSA stage of one anchor (local index ai) for one CTA. Every
 // early return is taken by all threads of the CTA together.
 // QB: the quality encoding the sums read (0: qualities unused, else 1, 2 or
-// 8 bits per quality); jb: 32-column blocks per warp (the MSA holds at most
-// 32 * jb * warps columns).
+// 8 bits per quality).
 template <int BLOCK, int QB, bool EMIT>
 __device__ __forceinline__ void
-msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, int jb,
+msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, const MsaGrid& grid,
            const uint32_t* __restrict__ cand_ids, const uint32_t* __restrict__ seg_off,
            const uint32_t* __restrict__ seg_cnt, const AlignRes* __restrict__ ares,
            CandRec* __restrict__ recs, const MsaOut& out, int* __restrict__ status) {
     constexpr int NWARP = BLOCK / 32;
-    const int MAXCOLS = 32 * jb * NWARP;
     extern __shared__ __align__(16) unsigned char dsm[];
-    __shared__ float s_qw[256];
-    // per warp: the staged rows meeting its column block, {row grid offset,
-    // first position - lane, length, weights}, and for 1- and 8-bit qualities
-    // the row's quality grid offset
-    __shared__ uint4 s_hits[NWARP][33];
-    __shared__ int s_hq[(QB == 1 || QB == 8) ? NWARP : 1][33];
-    __shared__ int s_blk;                    // next column block (persistent rows: warps take blocks in turn)
+    __shared__ float s_qw[QB == 8 ? 256 : 1];
     __shared__ float s_qwc[4];               // weight of a 1- or 2-bit quality code
-    __shared__ int s_beg[kStageMax], s_len[kStageMax];
-    __shared__ float s_w[kStageMax];
-    __shared__ uint32_t s_id[kStageMax];
-    __shared__ uint8_t s_fwd[kStageMax];
-    __shared__ int2 s_bl[kStageMax];         // {begin, length} of staged row k
-    __shared__ float s_wq[kStageMax][4];     // row weight * weight of a 1- or 2-bit quality code
-    __shared__ uint8_t s_alive[kStageMax];
-    __shared__ int s_red[NWARP][4];
-    __shared__ int s_vals[12];
+    // by slot (0: the anchor): shift, length, weight, id, orientation, weight
+    // * weight of a 1- or 2-bit quality code
+    __shared__ int16_t s_beg[kStageMax + 1], s_len[kStageMax + 1];
+    __shared__ float s_w[kStageMax + 1];
+    __shared__ uint32_t s_id[kStageMax + 1];
+    __shared__ uint8_t s_fwd[kStageMax + 1];
+    __shared__ __align__(16) float s_wq[kStageMax + 1][4];
+    // the rows of the sums in list order, {byte offset of the staged row,
+    // -shift, length, 16 * slot}, one entry of length 0 behind the last
+    __shared__ uint4 s_ent[kStageMax + 2];
+    __shared__ uint32_t s_dis[kMaxLen / 16];  // disputed columns, bit 30 - 2 * (position % 16)
+    __shared__ __align__(16) int s_diff[kMaxLen + 4]; // coverage changes by anchor position
+    __shared__ int s_red[NWARP + 1];
+    __shared__ int s_nd, s_sig, s_min, s_mincov, s_maxcov, s_bases, s_flags;
+    __shared__ float s_avg;
     __shared__ uint16_t s_dec[EMIT ? kMaxLen : 1];   // decision positions of the anchor (EMIT)
-    __shared__ __align__(16) float s_asup[kMaxLen];   // support of the anchor's columns, position order
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t a = first + ai;
     const uint32_t off = seg_off[ai], cnt = seg_cnt[ai];
     const int La = r.len[a];
     const int mlen = r.max_len;
-    constexpr bool useQ = QB != 0;
     char* aout = out.seq + (size_t)ai * mlen;
-    const int nstage = msa_stage_rows(r.seq_pitch, r.qual_pitch, QB);
-    const int rw = msa_slot_words(r.seq_pitch, r.qual_pitch, QB);   // words per staged row
-    // dynamic shared memory, each part 16-byte aligned (msa_smem_bytes)
-    uint16_t* s_aelem = (uint16_t*)dsm;                      // anchor row: base | quality char << 2
-    unsigned char* s_rawg = dsm + msa_round16((size_t)mlen * 2);
-    uint32_t* s_raw = (uint32_t*)(s_rawg + kStageGuard);     // [nstage][rw]
-    // per anchor column: column weight sum, consensus weight, weight of the
+    const int nstage = grid.rows, rw = grid.rw, G = grid.words, E = grid.edge, wpg = grid.wpg;
+    const int nwa = (La + 15) >> 4;
+    // dynamic shared memory (msa_smem_bytes)
+    uint32_t* s_raw = (uint32_t*)dsm;                        // [nstage + 1][rw]
+    float* s_sup = (float*)(dsm + msa_round16((size_t)(nstage + 1) * rw * 4));   // support by anchor position
+    ushort4* s_cnt4 = (ushort4*)((unsigned char*)s_sup + msa_round16((size_t)mlen * 4));   // counts A C G T (disputed)
+    // per anchor position: column weight sum, consensus weight, weight of the
     // anchor's base (EMIT only)
-    float* s_fw = (float*)(s_rawg + msa_raw_bytes(r.seq_pitch, r.qual_pitch, QB));
-    // per MSA column: counts of A C G T, support, coverage, consensus
-    ushort4* s_cnt4 = (ushort4*)((unsigned char*)s_fw + (EMIT ? msa_round16((size_t)3 * mlen * 4) : 0));
-    float* s_support = (float*)(s_cnt4 + MAXCOLS);
-    uint16_t* s_cov = (uint16_t*)(s_support + MAXCOLS);
-    uint8_t* s_cons = (uint8_t*)(s_cov + MAXCOLS);
-    auto cnt_of = [&](int col, int b) -> int {
-        const ushort4 c = s_cnt4[col];
-        return b == 0 ? c.x : b == 1 ? c.y : b == 2 ? c.z : c.w;
-    };
+    float* s_fw = (float*)((unsigned char*)s_cnt4 + (size_t)(mlen + (mlen & 1)) * 8);
+    uint16_t* s_cov = (uint16_t*)((unsigned char*)s_fw + (EMIT ? msa_round16((size_t)3 * mlen * 4) : 0));
+    int16_t* s_col = (int16_t*)((unsigned char*)s_cov + msa_round16((size_t)mlen * 2));   // columns of the sums
+    // per grid column: consensus | plain rule's base << 2 | anchor's base << 4
+    uint8_t* s_cons = (uint8_t*)s_col + msa_round16((size_t)16 * G * 2);
 
     if (cnt == 0) {
         if (tid == 0) { out.status[ai] = 0; out.nedits[ai] = 0; }
         return;
     }
-
-    auto block_sum4 = [&](int v0, int v1, int v2, int v3, int* res) {
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            v0 += __shfl_xor_sync(0xffffffffu, v0, d);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, d);
-            v2 += __shfl_xor_sync(0xffffffffu, v2, d);
-            v3 += __shfl_xor_sync(0xffffffffu, v3, d);
-        }
+    // block-wide rank of the threads with keep set (0/1); *tot gets their number
+    auto block_rank = [&](bool keep, int* tot) {
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
         __syncthreads();
-        if (lane == 0) { s_red[warp][0] = v0; s_red[warp][1] = v1; s_red[warp][2] = v2; s_red[warp][3] = v3; }
-        __syncthreads();
-        int t0 = 0, t1 = 0, t2 = 0, t3 = 0;
-#pragma unroll
-        for (int w = 0; w < NWARP; ++w) { t0 += s_red[w][0]; t1 += s_red[w][1]; t2 += s_red[w][2]; t3 += s_red[w][3]; }
-        res[0] = t0; res[1] = t1; res[2] = t2; res[3] = t3;
-    };
-    // block-wide exclusive scan of one value per thread; *tot gets the sum
-    auto block_scan = [&](int v, int* tot) {
-        int x = v;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, d);
-            if (lane >= d) x += y;
-        }
-        __syncthreads();
-        if (lane == 31) s_red[warp][0] = x;
+        if (lane == 0) s_red[warp] = __popc(m);
         __syncthreads();
         int pre = 0, all = 0;
 #pragma unroll
-        for (int w = 0; w < NWARP; ++w) { const int sv = s_red[w][0]; if (w < warp) pre += sv; all += sv; }
+        for (int w = 0; w < NWARP; ++w) { const int sv = s_red[w]; if (w < warp) pre += sv; all += sv; }
         *tot = all;
-        return pre + x - v;
+        return pre + __popc(m & ((1u << lane) - 1u));
     };
 
     // ---- quality weights (qualityscoreweights.hpp:12-44) ----
-    for (int i = tid; i < 256; i += BLOCK) s_qw[i] = c_qweight[i];
-    constexpr int qbits = QB;
+    if constexpr (QB == 8) for (int i = tid; i < 256; i += BLOCK) s_qw[i] = c_qweight[i];
     if (tid < 4) {
         // the characters a 2- or 1-bit code stands for (qualityscorecompression.hpp:121-145)
-        const uint32_t ch = qbits == 2 ? (tid == 0 ? '$' : tid == 1 ? '(' : tid == 2 ? '1' : '9')
-                                       : (tid == 1 ? '5' : '(');
+        const uint32_t ch = QB == 2 ? (tid == 0 ? '$' : tid == 1 ? '(' : tid == 2 ? '1' : '9')
+                                    : (tid == 1 ? '5' : '(');
         s_qwc[tid] = c_qweight[ch];
+        s_wq[0][tid] = c_qweight[ch];                        // the anchor's factor is 1
+    }
+    if (tid == 0) {
+        s_beg[0] = 0;
+        s_len[0] = (int16_t)La;
+        s_w[0] = 1.0f;
+        s_fwd[0] = 1;
+        s_id[0] = a;
     }
 
     // ---- alignment filters (corrector.hpp:982-1211), ordered compaction ----
     const float base = fmul_rn(o.estimated_errorrate, 1.0f);
     const float base2 = fmul_rn(2.0f, base), base3 = fmul_rn(3.0f, base), base4 = fmul_rn(4.0f, base);
-    int c0 = 0, c1 = 0, c2 = 0, n1 = 0;
     // the first candidate of each thread: its alignment, mismatch ratio, id
     // and length stay in registers for the compaction below (the id and
     // length loads overlap the counting)
@@ -989,15 +959,16 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
     float mr0 = 0.0f;
     uint32_t id0 = 0;
     int len0 = 0;
+    // counts below the three thresholds and of aligned candidates, 16 bits
+    // each (a list holds fewer than 2^14 candidates)
+    uint32_t c01 = 0, c23 = 0;
     for (uint32_t i = tid; i < cnt; i += BLOCK) {
         const AlignRes ar = ares[off + i];
         float mr = 0.0f;
         if (ar.orient != 3) {
-            n1++;
             mr = fdiv_rn((float)ar.nops, (float)ar.overlap);
-            c0 += mr < base2;
-            c1 += mr < base3;
-            c2 += mr < base4;
+            c01 += (mr < base2 ? 1u : 0u) + (mr < base3 ? 65536u : 0u);
+            c23 += (mr < base4 ? 1u : 0u) + 65536u;
         }
         if (i == (uint32_t)tid) {
             ar0 = ar;
@@ -1006,28 +977,47 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
             len0 = r.len[id0];
         }
     }
-    int red[4];
-    block_sum4(c0, c1, c2, n1, red);
-    if (red[3] == 0) {
+    c01 = __reduce_add_sync(0xffffffffu, c01);
+    c23 = __reduce_add_sync(0xffffffffu, c23);
+    __shared__ uint32_t s_cnt[NWARP][2];
+    if (lane == 0) { s_cnt[warp][0] = c01; s_cnt[warp][1] = c23; }
+    __syncthreads();
+    c01 = c23 = 0;
+#pragma unroll
+    for (int w = 0; w < NWARP; ++w) { c01 += s_cnt[w][0]; c23 += s_cnt[w][1]; }
+    if ((c23 >> 16) == 0) {
         if (tid == 0) { out.status[ai] = 0; out.nedits[ai] = 0; }
         return;
     }
     float thr = -3.402823466e+38f;
     {
         const float good = fmul_rn(o.estimated_coverage, o.m_coverage);
-        if (red[0] > 0 || red[1] > 0 || red[2] > 0) {
-            if ((float)red[0] >= good) thr = base2;
-            else if ((float)red[1] >= good) thr = base3;
-            else if ((float)red[2] >= good) thr = base4;
+        const int n2 = c01 & 0xFFFF, n3 = c01 >> 16, n4 = c23 & 0xFFFF;
+        if (n2 > 0 || n3 > 0 || n4 > 0) {
+            if ((float)n2 >= good) thr = base2;
+            else if ((float)n3 >= good) thr = base3;
+            else if ((float)n4 >= good) thr = base4;
         }
     }
+    // slot k of the staged rows
+    auto fill_slot = [&](int k, const CandRec& rec) {
+        s_beg[k] = rec.shift;
+        s_len[k] = (int16_t)rec.len;
+        s_w[k] = rec.weight;
+        s_fwd[k] = rec.orient == 1;
+        s_id[k] = rec.id;
+        if constexpr (QB == 1 || QB == 2)
+            *reinterpret_cast<float4*>(&s_wq[k][0]) =
+                make_float4(fmul_rn(rec.weight, s_qwc[0]), fmul_rn(rec.weight, s_qwc[1]),
+                            fmul_rn(rec.weight, s_qwc[2]), fmul_rn(rec.weight, s_qwc[3]));
+    };
     // every candidate fits the staged rows: the survivors' records go straight
     // to shared memory (else to the global records, staged chunk by chunk)
     const bool direct = cnt <= (uint32_t)nstage;
     int V = 0;
     for (uint32_t c = 0; c < cnt; c += BLOCK) {
         const uint32_t i = c + tid;
-        int keep = 0;
+        bool keep = false;
         AlignRes ar = ar0;
         float mr = mr0;
         if (i < cnt) {
@@ -1039,7 +1029,7 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                 keep = o.paired_end ? (ar.paired || mr < o.paired_filter_threshold) : (mr < thr);
         }
         int tot;
-        const int pre = block_scan(keep, &tot);
+        const int pre = block_rank(keep, &tot);
         if (keep) {
             CandRec rec;
             rec.id = c ? cand_ids[off + i] : id0;
@@ -1049,18 +1039,8 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
             rec.weight = fsub_rn(1.0f, __fsqrt_rn(fdiv_rn((float)ar.nops, fmul_rn((float)ar.overlap, o.max_error_rate))));
             rec.orient = ar.orient;
             const int k = V + pre;
-            if (direct) {
-                s_beg[k] = rec.shift;
-                s_len[k] = rec.len;
-                s_w[k] = rec.weight;
-                s_fwd[k] = rec.orient == 1;
-                s_id[k] = rec.id;
-                s_bl[k] = make_int2(rec.shift, rec.len);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) s_wq[k][q] = fmul_rn(rec.weight, s_qwc[q]);
-            } else {
-                recs[off + k] = rec;
-            }
+            if (direct) fill_slot(k + 1, rec);
+            else recs[off + k] = rec;
         }
         V += tot;
     }
@@ -1068,336 +1048,289 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
         if (tid == 0) { out.status[ai] = 0; out.nedits[ai] = 0; }
         return;
     }
-    __syncthreads();
 
-    // ---- anchor row ----
     const int sp = r.seq_pitch, qp = r.qual_pitch;
-    // quality character at position q of an encoded row (qualityscorecompression.hpp:121-145)
-    auto qual_char = [&](const uint32_t* row, int q) -> uint32_t {
-        if (qbits == 8) return (row[q >> 2] >> (8 * (q & 3))) & 0xFFu;
-        if (qbits == 2) {
-            const uint32_t b = (row[q >> 4] >> (30 - 2 * (q & 15))) & 3u;
-            return b == 0 ? '$' : b == 1 ? '(' : b == 2 ? '1' : '9';
-        }
-        return ((row[q >> 5] >> (31 - (q & 31))) & 1u) ? '5' : '(';
-    };
-    {
-        const uint32_t* arow = r.seq + (size_t)a * sp;
-        const uint32_t* aq = useQ ? r.qual + (size_t)a * qp : nullptr;
-        for (int p = tid; p < La; p += BLOCK) {
-            const uint32_t b = base_at(arow, p);
-            const uint32_t q = useQ ? qual_char(aq, p) : 0u;
-            s_aelem[p] = (uint16_t)(b | (q << 2));
-        }
-    }
-
-    // stage candidate rows [c, c+n) of recs into slots 0..n-1, realigned to
-    // the anchor's grid: the code at row position p of a row with shift s
-    // moves to anchor-relative position s + p, which lies in word
-    // (s + p) / 16 - s / 16 of the row's bases (floor divisions; 32 and 4
-    // codes per word for 1- and 8-bit qualities). Reverse-complement rows are
-    // turned into the alignment's orientation on the way (bases reversed and
-    // complemented, qualities reversed over the whole quality pitch:
-    // reverseQualitiesOfRCAlignments, corrector.hpp:1227-1239), so the column
-    // sums read every row forward, and a lane finds its column's code at the
-    // same bits of every row. A warp per row: lane j loads word j of the
-    // row's packed bases and of its quality words (RR rows of a warp in
-    // flight: two measured best, 21.6 ms per 1M anchors against 22.1 ms with
-    // one and 22.3 ms with four), then builds output word j from a window of
-    // them.
-    auto stage = [&](int c, int n, bool fill, auto RR) {
-        constexpr int R = decltype(RR)::value;
-        __syncthreads();
-        if (fill) {
-            for (int k = tid; k < n; k += BLOCK) {
-                const CandRec rc = recs[off + c + k];
-                s_beg[k] = rc.shift;                // relative to the anchor; abegin added per build
-                s_len[k] = rc.len;
-                s_w[k] = rc.weight;
-                s_fwd[k] = rc.orient == 1;
-                s_id[k] = rc.id;
-                s_bl[k] = make_int2(rc.shift, rc.len);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) s_wq[k][q] = fmul_rn(rc.weight, s_qwc[q]);
-            }
-            __syncthreads();
-        }
-        for (int k0 = warp * R; k0 < n; k0 += NWARP * R) {
-            uint32_t ms[R], mq0[R], mq1[R];
-#pragma unroll
-            for (int t = 0; t < R; ++t) {
-                ms[t] = mq0[t] = mq1[t] = 0u;
-                if (k0 + t < n) {
-                    const size_t id = s_id[k0 + t];
-                    if (lane < sp) ms[t] = __ldg(r.seq + id * sp + lane);
-                    if constexpr (useQ) {
-                        const uint32_t* qrow = r.qual + id * qp;
-                        if (lane < qp) mq0[t] = __ldg(qrow + lane);
-                        if constexpr (QB == 8) if (lane + 32 < qp) mq1[t] = __ldg(qrow + lane + 32);
-                    }
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < R; ++t) {
-                const int k = k0 + t;
-                if (k >= n) break;                           // warp-uniform
-                uint32_t* row = s_raw + k * rw;
-                const bool rev = !s_fwd[k];                  // warp-uniform
-                const int L = s_len[k], sft = s_beg[k];
-                const int o16 = sft & 15;
-                uint32_t ws = window2(ms[t], rev ? L - 16 - 16 * lane + o16 : 16 * lane - o16);
+    const uint32_t* arow = r.seq + (size_t)a * sp;
+    // Word g of slot k, a thread each: 16 codes from row position 16 (g - E) -
+    // shift on, reverse-complement rows turned into the alignment's
+    // orientation (bases reversed and complemented, qualities reversed over
+    // the whole quality pitch: reverseQualitiesOfRCAlignments,
+    // corrector.hpp:1227-1239). load: from the read storage (else the words
+    // are staged already); disputed columns are marked on the way.
+    // Slots k0 .. k0 + n - 1, or with list the slots of entries 1 .. n.
+    auto scan_words = [&](int n, int k0, bool load, bool list) {
+#pragma unroll 1
+        for (int idx = tid; idx < n * G; idx += BLOCK) {
+            const int e = G > 1 ? (int)__umulhi((uint32_t)idx, grid.magic) : idx, g = idx - e * G;
+            const int k = list ? (int)(s_ent[e + 1].w >> 4) : k0 + e;
+            const int p0 = 16 * (g - E);                     // anchor position of the word's first code
+            const int sft = s_beg[k], L = s_len[k];
+            const int lo = max(sft - p0, 0), hi = min(sft + L - p0, 16);
+            if (lo >= hi) continue;                          // the row does not reach the word
+            uint32_t* dst = s_raw + k * rw + g * wpg;
+            uint32_t ws;
+            if (load) {
+                const bool rev = !s_fwd[k];
+                const size_t id = s_id[k];
+                const int q0 = p0 - sft;
+                ws = window2(r.seq + id * sp, sp, rev ? L - 16 - q0 : q0);
                 if (rev) ws = ~rev2(ws);                     // reversed, complemented: A<->T, C<->G
                 if constexpr (QB == 2) {
-                    uint32_t wq = window2(mq0[t], rev ? mlen - 16 - 16 * lane + o16 : 16 * lane - o16);
+                    uint32_t wq = window2(r.qual + id * qp, qp, rev ? mlen - 16 - q0 : q0);
                     if (rev) wq = rev2(wq);
-                    if (lane <= (sp > qp ? sp : qp)) reinterpret_cast<uint2*>(row)[lane] = make_uint2(ws, wq);
+                    *reinterpret_cast<uint2*>(dst) = make_uint2(ws, wq);
                 } else {
-                    if (lane <= sp) row[lane] = ws;
+                    dst[0] = ws;
                     if constexpr (QB == 1) {
-                        const int o32 = sft & 31;
-                        uint32_t wq = window1(mq0[t], rev ? mlen - 32 - 32 * lane + o32 : 32 * lane - o32);
-                        if (rev) wq = __brev(wq);
-                        if (lane <= qp) row[sp + 1 + lane] = wq;
+                        uint32_t wq = window1(r.qual + id * qp, qp, rev ? mlen - 16 - q0 : q0);
+                        if (rev) wq = __brev(wq) << 16;
+                        dst[1] = wq;
                     } else if constexpr (QB == 8) {
-                        const int o4 = sft & 3;
 #pragma unroll
-                        for (int h = 0; h < 3; ++h) {
-                            const int j = lane + 32 * h;
-                            uint32_t wq = window8(mq0[t], mq1[t], rev ? mlen - 4 - 4 * j + o4 : 4 * j - o4);
+                        for (int h = 0; h < 4; ++h) {
+                            uint32_t wq = window8(r.qual + id * qp, qp, rev ? mlen - 4 - q0 - 4 * h : q0 + 4 * h);
                             if (rev) wq = __byte_perm(wq, 0u, 0x0123);
-                            if (j <= qp) row[sp + 1 + j] = wq;
+                            dst[1 + h] = wq;
                         }
                     }
                 }
+            } else {
+                ws = dst[0];
+            }
+            if (p0 >= 0 && p0 < La) {
+                const int end = min(hi, La - p0);
+                uint32_t d = ws ^ __ldg(arow + (p0 >> 4));
+                d = (d | (d >> 1)) & 0x55555555u & (0xFFFFFFFFu >> (2 * lo));
+                if (end < 16) d &= ~(0xFFFFFFFFu >> (2 * max(end, 0)));
+                if (d) atomicOr(&s_dis[p0 >> 4], d);
             }
         }
+    };
+    // entries of slots 1 .. n (and the anchor's, entry 0, when with_anchor)
+    auto put_entry = [&](int e, int k, int len) {
+        s_ent[e] = make_uint4((uint32_t)(k * rw * 4), (uint32_t)-(int)s_beg[k], (uint32_t)len, (uint32_t)k * 16u);
+    };
+    // a chunk of the global records into slots 1 .. n
+    auto stage_chunk = [&](int c, int n) {
+        __syncthreads();
+        for (int k = tid; k < n; k += BLOCK) {
+            fill_slot(k + 1, recs[off + c + k]);
+            put_entry(k + 1, k + 1, s_len[k + 1]);
+        }
+        if (tid == 0) put_entry(n + 1, 0, 0);
+        __syncthreads();
+        scan_words(n, 1, true, false);
         __syncthreads();
     };
-    // base (2-bit, in the candidate's aligned orientation) of staged row k at
-    // position p < s_len[k]
-    auto cand_base = [&](int k, int p) -> uint32_t {
-        const int sft = s_beg[k], q = sft + p;
-        const int wi = (q >> 4) - (sft >> 4);
-        const uint32_t w = s_raw[k * rw + (QB == 2 ? 2 * wi : wi)];
-        return (w >> (30 - 2 * (q & 15))) & 3u;
+    // base (2-bit, in the candidate's aligned orientation) of staged slot k at
+    // anchor position p
+    auto staged_base = [&](int k, int p) -> uint32_t {
+        return (s_raw[k * rw + ((p >> 4) + E) * wpg] >> (30 - 2 * (p & 15))) & 3u;
     };
     const bool persistent = V <= nstage;      // all rows stay staged across rebuilds
+    const int sigThr = f2i_rz(fmul_rn((float)o.coverage_int, 0.3f));
     int nalive = V;
-    if (persistent) {
-        stage(0, V, !direct, std::integral_constant<int, 2>{});
-        for (int k = tid; k < V; k += BLOCK) s_alive[k] = (uint8_t)k;
+    bool outside = false;                     // the sums of candidate correction's columns outside the anchor
+    bool hq = false;
+    int iter = 0;
+    if (persistent && !direct) {
+        __syncthreads();
+        for (int k = tid; k < V; k += BLOCK) fill_slot(k + 1, recs[off + k]);
     }
-    __syncthreads();
+    for (int i = tid; i < G * wpg; i += BLOCK) s_raw[i] = 0u;
 
-    int abegin = 0, aend = 0, ncols = 0;
-    bool allGood = false, hq = false;
-
-    for (int iter = 0;; ++iter) {
-        // ---- MSA geometry (build, msa.cpp:17-33) ----
-        int mn = 0, mx = La, sl = 0;                // sl: bases of the rows (roofline work)
-        if (persistent) {
-            for (int i = tid; i < nalive; i += BLOCK) {
-                const int k = s_alive[i];
-                mn = min(mn, s_beg[k]);
-                mx = max(mx, s_beg[k] + s_len[k]);
-                sl += s_len[k];
+    for (;;) {
+        int ncol;
+        if (!outside) {
+            // ---- disputed columns, coverage ----
+            for (int i = tid; i < kMaxLen + 4; i += BLOCK) s_diff[i] = 0;
+            if (tid < kMaxLen / 16) s_dis[tid] = tid == 0 && sigThr <= 0 ? 0x40000000u : 0u;   // counts of 0 are significant
+            if (tid == 0) { s_sig = 0x7fffffff; s_bases = 0; }
+            __syncthreads();
+            if (iter == 0) scan_words(1, 0, true, false);    // the anchor
+            int sl = 0;
+            auto add_cover = [&](int sft, int L) {
+                const int b = max(sft, 0), e = min(sft + L, La);
+                if (b < e) { atomicAdd(&s_diff[b], 1); atomicAdd(&s_diff[e], -1); }
+                sl += L;
+            };
+            if (persistent) {
+                scan_words(nalive, 1, iter == 0, iter > 0);
+                for (int i = tid; i < nalive; i += BLOCK) {
+                    const int k = iter == 0 ? i + 1 : (int)(s_ent[i + 1].w >> 4);
+                    if (iter == 0) put_entry(i + 1, k, s_len[k]);
+                    add_cover(s_beg[k], s_len[k]);
+                }
+                if (tid == 0) { put_entry(0, 0, La); put_entry(nalive + 1, 0, 0); }
+            } else {
+                for (int c = 0; c < nalive; c += nstage) {
+                    const int n = min(nstage, nalive - c);
+                    stage_chunk(c, n);
+                    for (int k = tid; k < n; k += BLOCK) add_cover(s_beg[k + 1], s_len[k + 1]);
+                }
+                if (tid == 0) {
+                    put_entry(0, 0, La);
+                    if (nalive == 0) put_entry(1, 0, 0);
+                }
             }
-        } else {
-            for (int k = tid; k < nalive; k += BLOCK) {
-                const CandRec rc = recs[off + k];
-                mn = min(mn, (int)rc.shift);
-                mx = max(mx, (int)rc.shift + (int)rc.len);
-                sl += rc.len;
+            if (out.elem_count) {
+                sl = __reduce_add_sync(0xffffffffu, sl);
+                if (lane == 0) atomicAdd(&s_bases, sl);
             }
-        }
+            __syncthreads();
+            if (warp == 0) {                                  // the list of disputed columns
+                uint32_t d = lane < nwa ? s_dis[lane] : 0u;
+                const int n = __popc(d);
+                int x = n;
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, d));
-            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
-            sl += __shfl_xor_sync(0xffffffffu, sl, d);
-        }
-        if (tid == 0) s_blk = 0;             // the previous build's sums are done (CTA barrier after them)
-        __syncthreads();
-        if (lane == 0) { s_red[warp][0] = mn; s_red[warp][1] = mx; s_red[warp][2] = sl; }
-        __syncthreads();
-        mn = 0; mx = La;
-        for (int w = 0; w < NWARP; ++w) { mn = min(mn, s_red[w][0]); mx = max(mx, s_red[w][1]); }
-        if (tid == 0 && out.elem_count) {
-            int tot = La;
-            for (int w = 0; w < NWARP; ++w) tot += s_red[w][2];
-            atomicAdd(out.elem_count, (unsigned long long)tot);
-            if (iter > 0 && out.rebuild_count) {
-                atomicAdd(out.rebuild_count, (unsigned long long)tot);
-                if (iter == 1) atomicAdd(out.rebuild_count + 1, 1ull);
+                for (int q = 1; q < 32; q <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, q); if (lane >= q) x += y; }
+                if (lane == 31) { s_nd = x; s_min = x < La ? __float_as_int(1.0f) : 0x7f7fffff; }
+                int at = x - n;
+                while (d) {
+                    const int bit = 31 - __clz(d);
+                    d &= ~(1u << bit);
+                    s_col[at++] = (int16_t)(16 * lane + (30 - bit) / 2);
+                }
+            } else if (warp == 1) {                           // coverage: prefix sums, 8 positions a lane
+                int v[8], sum = 0;
+                const int4 lo4 = *reinterpret_cast<const int4*>(&s_diff[8 * lane]);
+                const int4 hi4 = *reinterpret_cast<const int4*>(&s_diff[8 * lane + 4]);
+                v[0] = lo4.x; v[1] = lo4.y; v[2] = lo4.z; v[3] = lo4.w; v[4] = hi4.x; v[5] = hi4.y; v[6] = hi4.z; v[7] = hi4.w;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) { sum += v[q]; v[q] = sum; }
+                int x = sum;
+#pragma unroll
+                for (int q = 1; q < 32; q <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, q); if (lane >= q) x += y; }
+                const int before = x - sum + 1;               // the anchor itself
+                int mn = 0x7fffffff, mx = 0;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int p = 8 * lane + q, cv = before + v[q];
+                    if (p < La) {
+                        mn = min(mn, cv);
+                        mx = max(mx, cv);
+                        if constexpr (EMIT) s_cov[p] = (uint16_t)cv;
+                    }
+                }
+                mn = __reduce_min_sync(0xffffffffu, mn);
+                mx = __reduce_max_sync(0xffffffffu, mx);
+                if (lane == 0) { s_mincov = mn; s_maxcov = mx; }
+            } else {                                          // undisputed until summed
+                for (int p = tid - 64; p < La; p += BLOCK - 64) {
+                    const uint32_t ob = staged_base(0, p);
+                    s_cons[p + 16 * E] = (uint8_t)(ob * 21u);
+                    s_sup[p] = 1.0f;
+                }
             }
-        }
-        ncols = mx - mn;
-        abegin = -mn;
-        aend = abegin + La;
-        if (ncols > MAXCOLS) {
-            if (tid == 0) { atomicOr(status, kStatusColumns); out.status[ai] = 0; out.nedits[ai] = 0; }
-            return;
+            if (tid == 0 && out.elem_count) {
+                const unsigned long long tot = (unsigned long long)(La + s_bases);
+                atomicAdd(out.elem_count, tot);
+                if (iter > 0 && out.rebuild_count) {
+                    atomicAdd(out.rebuild_count, tot);
+                    if (iter == 1) atomicAdd(out.rebuild_count + 1, 1ull);
+                }
+            }
+            __syncthreads();
+            ncol = s_nd;
+        } else {
+            ncol = s_nd;
         }
 
         // ---- column sums (anchor first, then candidates in list order) and
-        //      consensus (findConsensus, msa.cpp:135-157): each warp takes one
-        //      32-column block at a time, lane = column ----
-        // persistent rows: the warps take the column blocks in turn from a
-        // shared counter (blocks differ in their row counts); rows staged in
-        // chunks: every warp runs its jb blocks (staging synchronises the CTA)
-        const int nblk = (ncols + 31) >> 5;
+        //      consensus (findConsensus, msa.cpp:135-157): 32 listed columns
+        //      a warp, lane = column ----
+        int mism = 0;
+        const int nblk = (ncol + 31) >> 5;
+        const int nchunk = persistent ? 1 : max(1, (nalive + nstage - 1) / nstage);
 #pragma unroll 1
-        for (int j = 0;; ++j) {
-            int blk;
-            if (persistent) {
-                if (lane == 0) blk = atomicAdd(&s_blk, 1);
-                blk = __shfl_sync(0xffffffffu, blk, 0);
-                if (blk >= nblk) break;
-            } else {
-                if (j >= jb) break;
-                blk = warp + NWARP * j;
-            }
-            const int c0 = 32 * blk;
-            const int col = c0 + lane;
-            const bool active = c0 < ncols;                  // warp-uniform
+        for (int b0 = 0; b0 < nblk; b0 += NWARP) {
+            const int ci = 32 * (b0 + warp) + lane;
+            const bool act = ci < ncol;
+            const int p = act ? s_col[ci] : 0;               // anchor position of the lane's column
             uint32_t cAC = 0u, cGT = 0u;                     // 16-bit counts: A | C << 16, G | T << 16
-            uint32_t c8 = 0u;           // the chunk's 8-bit counts A | C << 8 | G << 16 | T << 24
             float wA = 0.0f, wC = 0.0f, wG = 0.0f, wT = 0.0f;
-            // a chunk adds at most 128 rows and the anchor: its 8-bit counts
-            // cannot overflow before they are moved to the 16-bit ones
-            auto flush = [&]() {
-                cAC += (c8 & 0xFFu) | ((c8 & 0xFF00u) << 8);
-                cGT += ((c8 >> 16) & 0xFFu) | ((c8 >> 24) << 16);
-                c8 = 0u;
-            };
-            {
-                const int p = col - abegin;
-                if (active && p >= 0 && p < La) {
-                    const uint32_t e = s_aelem[p];
-                    msa_add8(wA, wC, wG, wT, c8, (e & 3u) << 3, useQ ? s_qw[e >> 2] : 1.0f, 0, 1);   // factor 1.0f
-                }
-            }
-            // staged rows (slot list[i], or slot i) meeting this block, in
-            // list order: per chunk of 32 rows the warp lists the rows that
-            // meet the block (ballot, order kept) as {grid origin of the row
-            // in bytes, first position - lane, length, weights}; two listed
-            // rows load together, then add in order (measured: 21.6 ms per
-            // 1M anchors against 22.3 ms with four and 24.3 ms with one). The
-            // last listed row is repeated past the list with length 0: a pair
-            // reads it there, in bounds, and adds nothing.
-            auto run_rows = [&](const uint8_t* list, int nrows) {
-                // this lane's column on the anchor's grid: the word of every
-                // staged row that holds it (byte offset, relative to the
-                // row's grid origin) and its bits there, as rotations that
-                // bring the base to bits 3-4 (base * 8) and the quality code
-                // to bits 2-3 (2-bit) or bit 2 (1-bit), i.e. the byte offset
-                // of its weight
-                const int q = col - abegin;
-                const int qsh = 30 - 2 * (q & 15);
-                const uint32_t rb8 = (uint32_t)(qsh + 29) & 31u;
-                const int loff = (q >> 4) * (QB == 2 ? 8 : 4);
-                uint32_t rq = 0u;
-                int qoff = 0;
-                if constexpr (QB == 2) rq = (uint32_t)(qsh + 30) & 31u;
-                if constexpr (QB == 1) { rq = (uint32_t)(31 - (q & 31) + 30) & 31u; qoff = (q >> 5) * 4; }
-                if constexpr (QB == 8) { rq = 8u * (uint32_t)(q & 3); qoff = (q >> 2) * 4; }
-                const unsigned char* rawb = reinterpret_cast<const unsigned char*>(s_raw);
-                const unsigned char* wqb = reinterpret_cast<const unsigned char*>(&s_wq[0][0]);
-                for (int i0 = 0; i0 < nrows; i0 += 32) {
-                    bool hit = false;
-                    uint4 ent = make_uint4(0u, 0u, 0u, 0u);
-                    int hq = 0;
-                    if (i0 + lane < nrows) {
-                        const int k = list ? list[i0 + lane] : i0 + lane;
-                        const int2 bl = s_bl[k];
-                        const int cb = abegin + bl.x;
-                        hit = cb < c0 + 32 && cb + bl.y > c0;
-                        ent.x = (uint32_t)(k * rw * 4 - (bl.x >> 4) * (QB == 2 ? 8 : 4));
-                        ent.y = (uint32_t)(c0 - cb);
-                        ent.z = (uint32_t)bl.y;
-                        ent.w = (QB == 1 || QB == 2) ? (uint32_t)k * 16u : __float_as_uint(s_w[k]);
-                        if constexpr (QB == 1) hq = (k * rw + sp + 1 - (bl.x >> 5)) * 4;
-                        if constexpr (QB == 8) hq = (k * rw + sp + 1 - (bl.x >> 2)) * 4;
-                    }
-                    const unsigned m = __ballot_sync(0xffffffffu, hit);
-                    const int nh = __popc(m);
-                    if (hit) {
-                        const int pos = __popc(m & ((1u << lane) - 1u));
-                        s_hits[warp][pos] = ent;
-                        if constexpr (QB == 1 || QB == 8) s_hq[warp][pos] = hq;
-                        if (pos == nh - 1) {
-                            s_hits[warp][pos + 1] = make_uint4(ent.x, ent.y, 0u, ent.w);
-                            if constexpr (QB == 1 || QB == 8) s_hq[warp][pos + 1] = hq;
-                        }
-                    }
-                    __syncwarp();
-                    for (int h0 = 0; h0 < nh; h0 += 2) {
-                        uint32_t bb[2];
-                        float ww[2];
-                        int pp[2], ll[2];
-#pragma unroll
-                        for (int u = 0; u < 2; ++u) {
-                            const uint4 e = s_hits[warp][h0 + u];
-                            const unsigned char* wp = rawb + ((int)e.x + loff);
-                            uint32_t sw, qv = 0u;
-                            if constexpr (QB == 2) {
-                                const uint2 t2 = *reinterpret_cast<const uint2*>(wp);
-                                sw = t2.x;
-                                qv = t2.y;
-                            } else {
-                                sw = *reinterpret_cast<const uint32_t*>(wp);
-                                if constexpr (QB == 1 || QB == 8)
-                                    qv = *reinterpret_cast<const uint32_t*>(rawb + (s_hq[warp][h0 + u] + qoff));
-                            }
-                            bb[u] = __funnelshift_r(sw, sw, rb8) & 24u;
-                            if constexpr (QB == 0) ww[u] = __uint_as_float(e.w);
-                            else if constexpr (QB == 2)
-                                ww[u] = *reinterpret_cast<const float*>(wqb + (e.w + (__funnelshift_r(qv, qv, rq) & 12u)));
-                            else if constexpr (QB == 1)
-                                ww[u] = *reinterpret_cast<const float*>(wqb + (e.w + (__funnelshift_r(qv, qv, rq) & 4u)));
-                            else ww[u] = fmul_rn(__uint_as_float(e.w), s_qw[(qv >> rq) & 0xFFu]);
-                            pp[u] = lane + (int)e.y;
-                            ll[u] = (int)e.z;
-                        }
-#pragma unroll
-                        for (int u = 0; u < 2; ++u) msa_add8(wA, wC, wG, wT, c8, bb[u], ww[u], pp[u], ll[u]);
-                    }
-                    __syncwarp();
-                }
-            };
-            // persistent rows are one chunk; with more rows than fit, each
-            // chunk is staged (by all warps) per block
-            const int nchunk = persistent ? 1 : (nalive + nstage - 1) / nstage;
+            // the lane's word in every staged row (byte offset) and its bits
+            // there, as rotations that bring the base to bits 3-4 (base * 8)
+            // and the quality code to bits 2-3 (2-bit) or bit 2 (1-bit), i.e.
+            // the byte offset of its weight
+            const int gw = (p >> 4) + E;
+            const uint32_t rb8 = (uint32_t)(59 - 2 * (p & 15)) & 31u;
+            const int loff = gw * wpg * 4;
+            uint32_t rq = 0u;
+            int qoff = 0;
+            if constexpr (QB == 2) rq = (uint32_t)(60 - 2 * (p & 15)) & 31u;
+            if constexpr (QB == 1) rq = (uint32_t)(61 - (p & 15)) & 31u;
+            if constexpr (QB == 8) { rq = 8u * (uint32_t)(p & 3); qoff = 4 + 4 * ((p & 15) >> 2); }
+            const unsigned char* rawb = reinterpret_cast<const unsigned char*>(s_raw) + loff;
+            const unsigned char* wqb = reinterpret_cast<const unsigned char*>(&s_wq[0][0]);
+#pragma unroll 1
             for (int ch = 0; ch < nchunk; ++ch) {
                 int n = nalive;
                 if (!persistent) {
                     n = min(nstage, nalive - ch * nstage);
-                    stage(ch * nstage, n, true, std::integral_constant<int, 1>{});
+                    if (nchunk > 1) stage_chunk(ch * nstage, n);
                 }
-                if (active) run_rows(persistent ? s_alive : nullptr, n);
-                flush();
+                if (32 * (b0 + warp) >= ncol) continue;      // warp-uniform (no barrier below)
+                uint32_t c8 = 0u;       // the chunk's 8-bit counts A | C << 8 | G << 16 | T << 24: at most 129 rows
+#pragma unroll 1
+                for (int i = ch == 0 ? 0 : 1; i <= n; i += 2) {
+                    uint32_t bb[2];
+                    float ww[2];
+                    int pp[2], ll[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const uint4 e = s_ent[i + u];
+                        const unsigned char* wp = rawb + e.x;
+                        uint32_t sw, qv = 0u;
+                        if constexpr (QB == 2) {
+                            const uint2 t2 = *reinterpret_cast<const uint2*>(wp);
+                            sw = t2.x;
+                            qv = t2.y;
+                        } else {
+                            sw = *reinterpret_cast<const uint32_t*>(wp);
+                            if constexpr (QB == 1) qv = *reinterpret_cast<const uint32_t*>(wp + 4);
+                            if constexpr (QB == 8) qv = *reinterpret_cast<const uint32_t*>(wp + qoff);
+                        }
+                        bb[u] = __funnelshift_r(sw, sw, rb8) & 24u;
+                        if constexpr (QB == 0) ww[u] = s_w[e.w >> 4];
+                        else if constexpr (QB == 2)
+                            ww[u] = *reinterpret_cast<const float*>(wqb + (e.w + (__funnelshift_r(qv, qv, rq) & 12u)));
+                        else if constexpr (QB == 1)
+                            ww[u] = *reinterpret_cast<const float*>(wqb + (e.w + (__funnelshift_r(qv, qv, rq) & 4u)));
+                        else ww[u] = fmul_rn(s_w[e.w >> 4], s_qw[(qv >> rq) & 0xFFu]);
+                        pp[u] = p + (int)e.y;
+                        ll[u] = (int)e.z;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) msa_add8(wA, wC, wG, wT, c8, bb[u], ww[u], pp[u], ll[u]);
+                }
+                cAC += (c8 & 0xFFu) | ((c8 & 0xFF00u) << 8);
+                cGT += ((c8 >> 16) & 0xFFu) | ((c8 >> 24) << 16);
             }
-            if (active && col < ncols) {
-                uint8_t cs = 0; float cw = wA;
+            if (act) {
+                uint32_t cs = 0; float cw = wA;
                 if (wC > cw) { cs = 1; cw = wC; }
                 if (wG > cw) { cs = 2; cw = wG; }
                 if (wT > cw) { cs = 3; cw = wT; }
-                const float colw = __fadd_rn(__fadd_rn(__fadd_rn(wA, wC), wG), wT);
-                s_cons[col] = cs;
-                const float sup = fdiv_rn(cw, colw);
-                s_support[col] = sup;
-                {
-                    const int p = col - abegin;
-                    if (p >= 0 && p < La) s_asup[p] = sup;
-                }
-                const uint32_t nA = cAC & 0xFFFFu, nC = cAC >> 16;
-                const uint32_t nG = cGT & 0xFFFFu, nT = cGT >> 16;
-                s_cov[col] = (uint16_t)(nA + nC + nG + nT);
-                s_cnt4[col] = make_ushort4((uint16_t)nA, (uint16_t)nC, (uint16_t)nG, (uint16_t)nT);
-                if constexpr (EMIT) {
-                    const int p = col - abegin;
-                    if (p >= 0 && p < La) {
-                        const uint32_t ob = s_aelem[p] & 3u;
+                if (outside) {
+                    s_cons[p + 16 * E] = (uint8_t)cs;
+                } else {
+                    const float colw = __fadd_rn(__fadd_rn(__fadd_rn(wA, wC), wG), wT);
+                    const float sup = fdiv_rn(cw, colw);
+                    const uint32_t nA = cAC & 0xFFFFu, nC = cAC >> 16, nG = cGT & 0xFFFFu, nT = cGT >> 16;
+                    const uint32_t ob = staged_base(0, p);
+                    // origCoverages: count of the anchor's base
+                    const uint32_t oc = ob == 0 ? nA : ob == 1 ? nC : ob == 2 ? nG : nT;
+                    const uint32_t rule = sup > 0.90f && oc <= 2u ? cs : ob;
+                    s_cons[p + 16 * E] = (uint8_t)(cs | rule << 2 | ob << 4);
+                    s_sup[p] = sup;
+                    s_cnt4[p] = make_ushort4((uint16_t)nA, (uint16_t)nC, (uint16_t)nG, (uint16_t)nT);
+                    mism |= cs != ob;
+                    const bool sig = (cs != 0 && sigThr <= (int)nA) || (cs != 1 && sigThr <= (int)nC) ||
+                                     (cs != 2 && sigThr <= (int)nG) || (cs != 3 && sigThr <= (int)nT);
+                    if (sig) atomicMin(&s_sig, p);
+                    atomicMin(&s_min, __float_as_int(sup));   // supports are positive
+                    if constexpr (EMIT) {
                         s_fw[p] = colw;
                         s_fw[mlen + p] = cw;
                         s_fw[2 * mlen + p] = ob == 0 ? wA : ob == 1 ? wC : ob == 2 ? wG : wT;
@@ -1405,131 +1338,98 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                 }
             }
         }
-        __syncthreads();
+        mism = __syncthreads_or(mism);
+        if (outside) break;
 
-        if (iter >= 5) break;
         // ---- refinement: findCandidatesOfDifferentRegion (msa.cpp:532-734) ----
-        if (tid == 0) s_vals[1] = 0x7fffffff;
-        int mism = 0;
-        for (int p = tid; p < La; p += BLOCK) mism |= (s_aelem[p] & 3u) != s_cons[abegin + p];
-        if (__syncthreads_or(mism) == 0) break;
-        const int sigThr = f2i_rz(fmul_rn((float)o.coverage_int, 0.3f));
-        for (int p = tid; p < La; p += BLOCK) {
-            const int col = abegin + p;
-            const int cs = s_cons[col];
-            bool sig = false;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) sig |= (b != cs && sigThr <= cnt_of(col, b));
-            if (sig) atomicMin(&s_vals[1], col);
-        }
-        __syncthreads();
-        const int col = s_vals[1];
-        if (col == 0x7fffffff) break;
-        int foundBase = -1;                   // the last qualifying base index wins (:591-601)
-        {
-            const int cs = s_cons[col];
-            for (int b = 0; b < 4; ++b) if (b != cs && sigThr <= cnt_of(col, b)) foundBase = b;
-        }
-        const int orig = s_aelem[col - abegin] & 3u;
-        const bool keepMatching = orig == foundBase;
-        // per candidate: remove? (discard_rows :622-665); veto by weight >= 0.90 (:672-689)
-        auto removes = [&](int b) { return keepMatching ? (b != foundBase) : (b == foundBase); };
-        int nrem = 0, veto = 0;
-        if (persistent) {
+        const int col = s_sig;                               // first column with a significant other base
+        if (iter < 5 && mism && col != 0x7fffffff) {
+            int foundBase = -1;               // the last qualifying base index wins (:591-601)
+            {
+                const ushort4 c4 = s_cnt4[col];
+                const int cs = s_cons[col + 16 * E] & 3;
+                if (cs != 0 && sigThr <= (int)c4.x) foundBase = 0;
+                if (cs != 1 && sigThr <= (int)c4.y) foundBase = 1;
+                if (cs != 2 && sigThr <= (int)c4.z) foundBase = 2;
+                if (cs != 3 && sigThr <= (int)c4.w) foundBase = 3;
+            }
+            const bool keepMatching = (int)staged_base(0, col) == foundBase;
+            // per candidate: remove? (discard_rows :622-665); veto by weight >= 0.90 (:672-689)
+            auto removes = [&](int b) { return keepMatching ? (b != foundBase) : (b == foundBase); };
+            auto record_removed = [&](const CandRec& rc) {
+                const int q = col - rc.shift;
+                if (q < 0 || q >= (int)rc.len) return false;
+                const uint32_t* row = r.seq + (size_t)rc.id * sp;
+                return removes(rc.orient == 1 ? (int)base_at(row, q) : (int)(base_at(row, rc.len - 1 - q) ^ 3u));
+            };
+            auto slot_removed = [&](int k) {
+                const int q = col - s_beg[k];
+                return q >= 0 && q < s_len[k] && removes((int)staged_base(k, col));
+            };
+            int nrem = 0, veto = 0;
             for (int i = tid; i < nalive; i += BLOCK) {
-                const int k = s_alive[i];
-                const int rb = abegin + s_beg[k], re = rb + s_len[k];
-                const int rem = (col >= rb && col < re) ? removes((int)cand_base(k, col - rb)) : 0;
-                nrem += rem;
-                veto |= rem && s_w[k] >= 0.90f;
-            }
-        } else {
-            for (int k = tid; k < nalive; k += BLOCK) {
-                const CandRec rc = recs[off + k];
-                const int rb = abegin + rc.shift, re = rb + rc.len;
-                int rem = 0;
-                if (col >= rb && col < re) {
-                    const int p = col - rb;
-                    const uint32_t* row = r.seq + (size_t)rc.id * sp;
-                    rem = removes(rc.orient == 1 ? (int)base_at(row, p) : (int)(base_at(row, rc.len - 1 - p) ^ 3u));
-                }
-                nrem += rem;
-                veto |= rem && rc.weight >= 0.90f;
-            }
-        }
-        const int anyVeto = __syncthreads_or(veto);
-        const int anyRem = __syncthreads_or(nrem);
-        if (anyVeto || !anyRem) break;        // nothing removed: the rebuilt MSA would be identical
-        // ordered compaction of the survivors
-        int newV = 0;
-        for (int c = 0; c < nalive; c += BLOCK) {
-            const int i = c + tid;
-            int keep = 0, k = 0;
-            CandRec rc;
-            if (i < nalive) {
+                bool rem;
+                float w;
                 if (persistent) {
-                    k = s_alive[i];
-                    const int rb = abegin + s_beg[k], re = rb + s_len[k];
-                    keep = !((col >= rb && col < re) && removes((int)cand_base(k, col - rb)));
+                    const int k = (int)(s_ent[i + 1].w >> 4);
+                    rem = slot_removed(k);
+                    w = s_w[k];
                 } else {
-                    rc = recs[off + i];
-                    const int rb = abegin + rc.shift, re = rb + rc.len;
-                    keep = 1;
-                    if (col >= rb && col < re) {
-                        const int p = col - rb;
-                        const uint32_t* row = r.seq + (size_t)rc.id * sp;
-                        keep = !removes(rc.orient == 1 ? (int)base_at(row, p) : (int)(base_at(row, rc.len - 1 - p) ^ 3u));
-                    }
+                    const CandRec rc = recs[off + i];
+                    rem = record_removed(rc);
+                    w = rc.weight;
                 }
+                nrem |= rem;
+                veto |= rem && w >= 0.90f;
             }
-            int tot;
-            const int pre = block_scan(keep, &tot);
-            __syncthreads();
-            if (keep) {
-                if (persistent) s_alive[newV + pre] = (uint8_t)k;
-                else recs[off + newV + pre] = rc;
+            const int anyVeto = __syncthreads_or(veto);
+            const int anyRem = __syncthreads_or(nrem);
+            if (!anyVeto && anyRem) {             // else the rebuilt MSA would be identical
+                // ordered compaction of the survivors
+                int newV = 0;
+                for (int c = 0; c < nalive; c += BLOCK) {
+                    const int i = c + tid;
+                    bool keep = false;
+                    uint4 ent = make_uint4(0u, 0u, 0u, 0u);
+                    CandRec rc{};
+                    if (i < nalive) {
+                        if (persistent) { ent = s_ent[i + 1]; keep = !slot_removed((int)(ent.w >> 4)); }
+                        else { rc = recs[off + i]; keep = !record_removed(rc); }
+                    }
+                    int tot;
+                    const int pre = block_rank(keep, &tot);
+                    __syncthreads();
+                    if (keep) {
+                        if (persistent) s_ent[1 + newV + pre] = ent;
+                        else recs[off + newV + pre] = rc;
+                    }
+                    newV += tot;
+                    __syncthreads();
+                }
+                nalive = newV;
+                ++iter;
+                __syncthreads();
+                continue;
             }
-            newV += tot;
-            __syncthreads();
         }
-        nalive = newV;
-        __syncthreads();
-    }
-    V = nalive;
 
-    // ---- MSA properties (getMSAProperties, msa.cpp:304-376) ----
-    {
-        float mnS = 3.402823466e+38f;
-        int mnC = 0x7fffffff;
-        for (int p = tid; p < La; p += BLOCK) {
-            mnS = fminf(mnS, s_support[abegin + p]);
-            mnC = min(mnC, (int)s_cov[abegin + p]);
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            mnS = fminf(mnS, __shfl_xor_sync(0xffffffffu, mnS, d));
-            mnC = min(mnC, __shfl_xor_sync(0xffffffffu, mnC, d));
-        }
-        __syncthreads();
-        if (lane == 0) { s_red[warp][0] = __float_as_int(mnS); s_red[warp][1] = mnC; }
-        __syncthreads();
+        // ---- MSA properties (getMSAProperties, msa.cpp:304-376) ----
         if (warp == 0) {
-            float minSup = 3.402823466e+38f;
-            int minCov = 0x7fffffff;
-            for (int w = 0; w < NWARP; ++w) { minSup = fminf(minSup, __int_as_float(s_red[w][0])); minCov = min(minCov, s_red[w][1]); }
             // std::accumulate order: one serial chain of IEEE adds (lane 0),
             // the supports read four at a time
             float sum = 0.0f;
             if (lane == 0) {
-                const float4* v4 = reinterpret_cast<const float4*>(s_asup);
+                const float4* v4 = reinterpret_cast<const float4*>(s_sup);
                 int p = 0;
                 for (; p + 4 <= La; p += 4) {
                     const float4 v = v4[p >> 2];
                     sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
                 }
-                for (; p < La; ++p) sum = __fadd_rn(sum, s_asup[p]);
+                for (; p < La; ++p) sum = __fadd_rn(sum, s_sup[p]);
             }
             sum = __shfl_sync(0xffffffffu, sum, 0);
+            const float minSup = __int_as_float(s_min);
+            const int minCov = s_mincov;
             const float avgSup = fdiv_rn(sum, (float)La);
             const float e = o.estimated_errorrate;
             const float avgThr = fsub_rn(1.0f, fmul_rn(1.0f, e));
@@ -1557,158 +1457,178 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                 isHQ = fgeq((float)minCov, covThr) && fleq((float)smallest, fmul_rn((float)pct, 0.5f));
             }
             if (lane == 0) {
-                s_vals[10] = 0;                  // decision positions listed (EMIT)
-                s_vals[4] = good;
-                s_vals[5] = isHQ;
-                s_vals[6] = __float_as_int(avgSup);
-                s_vals[7] = __float_as_int(minSup);
-                s_vals[8] = minCov;
+                s_nd = 0;                     // decision positions listed (EMIT)
+                s_flags = (good ? 1 : 0) | (isHQ ? 2 : 0);
+                s_avg = avgSup;
+                s_red[NWARP] = 0;
             }
         }
         __syncthreads();
-        allGood = s_vals[4];
-        hq = s_vals[5];
-    }
+        const bool allGood = s_flags & 1;
+        hq = s_flags & 2;
 
-    // ---- anchor correction (getCorrectedAnchor, msa.cpp:379-453) ----
-    if (V == 0) {
-        if (tid == 0) { out.status[ai] = 0; out.nedits[ai] = 0; }
-        return;   // nCandidates == 0: not corrected; no candidate corrections either
-    }
-    int diffs = 0;
-    for (int p = tid; p < La; p += BLOCK) {
-        const int col = abegin + p;
-        const uint32_t ob = s_aelem[p] & 3u;
-        uint32_t cb;
-        if (allGood) cb = s_cons[col];
-        else {
-            const int oc = cnt_of(col, ob);   // origCoverages: count of the anchor's base
-            cb = (s_support[col] > 0.90f && oc <= 2) ? s_cons[col] : ob;
+        // ---- anchor correction (getCorrectedAnchor, msa.cpp:379-453) ----
+        if (nalive == 0) {
+            if (tid == 0) { out.status[ai] = 0; out.nedits[ai] = 0; }
+            return;   // nCandidates == 0: not corrected; no candidate corrections either
         }
-        aout[p] = "ACGT"[cb];
-        diffs += cb != ob;
-    }
-    int rr[4];
-    block_sum4(diffs, 0, 0, 0, rr);
-    if (tid == 0) {
-        const int nd = rr[0];
-        const bool useEdits = !r.ambig[a] && nd <= La / 7;
-        out.status[ai] = (uint8_t)(1 | (hq ? 2 : 0) | (useEdits ? 4 : 0));
-        out.nedits[ai] = useEdits ? nd : 0;
-    }
+        int diffs = 0;
+        for (int p = tid; p < La; p += BLOCK) {
+            const uint32_t e = s_cons[p + 16 * E];
+            const uint32_t cb = allGood ? e & 3u : (e >> 2) & 3u;
+            aout[p] = "ACGT"[cb];
+            diffs += cb != e >> 4;
+        }
+        diffs = __reduce_add_sync(0xffffffffu, diffs);
+        if (lane == 0 && diffs) atomicAdd(&s_red[NWARP], diffs);
+        __syncthreads();
+        if (tid == 0) {
+            const int nd = s_red[NWARP];
+            const bool useEdits = !r.ambig[a] && nd <= La / 7;
+            out.status[ai] = (uint8_t)(1 | (hq ? 2 : 0) | (useEdits ? 4 : 0));
+            out.nedits[ai] = useEdits ? nd : 0;
+        }
 
-    // ---- decision columns (correctAnchorClf, corrector.hpp:1448-1472) ----
-    // Non-HQ MSAs only: each anchor position whose base differs from the
-    // consensus (and whose column reaches clf_min_coverage) becomes a row of
-    // 24 features. The plain rule's base stays in aout; with the network
-    // deciding, k_clf_apply overwrites it from the row's logit.
-    if constexpr (EMIT) {
-        if (!hq) {
-            // the decision positions are listed first (any order: rows are
-            // appended through a global counter), so that their features are
-            // computed by consecutive threads instead of by the warps that
-            // happen to hold one
-            int nm = 0, mxc = 0;
-            for (int p = tid; p < La; p += BLOCK) {
-                const int col = abegin + p;
-                const bool mis = (s_aelem[p] & 3u) != s_cons[col];
-                nm += mis;
-                mxc = max(mxc, (int)s_cov[col]);
-                if (mis && (int)s_cov[col] >= o.clf_min_coverage) s_dec[atomicAdd(&s_vals[10], 1)] = (uint16_t)p;
-            }
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) {
-                nm += __shfl_xor_sync(0xffffffffu, nm, d);
-                mxc = max(mxc, __shfl_xor_sync(0xffffffffu, mxc, d));
-            }
-            __syncthreads();
-            if (lane == 0) { s_red[warp][0] = nm; s_red[warp][1] = mxc; }
-            __syncthreads();
-            int nmis = 0, maxCov = 0;
-#pragma unroll
-            for (int w = 0; w < NWARP; ++w) { nmis += s_red[w][0]; maxCov = max(maxCov, s_red[w][1]); }
-            const float avgSup = __int_as_float(s_vals[6]), minSup = __int_as_float(s_vals[7]);
-            const int minCov = s_vals[8];
-            const float E = o.estimated_coverage;
-            const int ndec = s_vals[10];
-            for (int i = tid; i < ndec; i += BLOCK) {
-                const int p = s_dec[i];
-                const int col = abegin + p;
-                const uint32_t ob = s_aelem[p] & 3u, cb = s_cons[col];
-                const float cov = (float)s_cov[col];
-                const int oc = cnt_of(col, ob), cc = cnt_of(col, cb);
-                const float wsum = s_fw[p], wc = s_fw[mlen + p], wo = s_fw[2 * mlen + p];
-                float x[kNumFeatures];
-                x[0] = fdiv_rn((float)oc, cov);
-                x[1] = fdiv_rn(wo, wsum);
-                x[2] = fdiv_rn(wo, (float)oc);
-                x[3] = fdiv_rn((float)cc, cov);
-                x[4] = s_support[col];
-                x[5] = fdiv_rn(wc, (float)cc);
-                x[6] = fdiv_rn(wsum, cov);
-                x[7] = fdiv_rn(cov, E);
-                x[8] = fdiv_rn(wsum, E);
-                x[9] = avgSup;
-                x[10] = minSup;
-                x[11] = fdiv_rn((float)maxCov, E);
-                x[12] = fdiv_rn((float)minCov, E);
-                x[13] = useQ ? s_qw[s_aelem[p] >> 2] : 1.0f;
-                x[14] = fdiv_rn((float)min(p, La - 1 - p), (float)La);
-                x[15] = fdiv_rn(fsub_rn(fsub_rn(wsum, wc), wo), wsum);
-                const int lo = max(p - 3, 0), hi = min(p + 3, La - 1);
-                float ssum = 0.0f, smin = s_support[abegin + lo], qsum = 0.0f;
-                for (int q = lo; q <= hi; ++q) {
-                    const float sv = s_support[abegin + q];
-                    ssum = __fadd_rn(ssum, sv);
-                    if (sv < smin) smin = sv;
-                    qsum = __fadd_rn(qsum, useQ ? s_qw[s_aelem[q] >> 2] : 1.0f);
+        // ---- decision columns (correctAnchorClf, corrector.hpp:1448-1472) ----
+        // Non-HQ MSAs only: each anchor position whose base differs from the
+        // consensus (and whose column reaches clf_min_coverage) becomes a row of
+        // 24 features. The plain rule's base stays in aout; with the network
+        // deciding, k_clf_apply overwrites it from the row's logit.
+        if constexpr (EMIT) {
+            if (!hq) {
+                // the decision positions are listed first (any order: rows are
+                // appended through a global counter), so that their features are
+                // computed by consecutive threads instead of by the warps that
+                // happen to hold one
+                auto mismatch = [&](int p) { const uint32_t e = s_cons[p + 16 * E]; return (e & 3u) != e >> 4; };
+                // the anchor's quality weight at position q
+                auto anchor_weight = [&](int q) -> float {
+                    const uint32_t* w = s_raw + ((q >> 4) + E) * wpg;
+                    if constexpr (QB == 0) return 1.0f;
+                    else if constexpr (QB == 2) return s_wq[0][(w[1] >> (30 - 2 * (q & 15))) & 3u];
+                    else if constexpr (QB == 1) return s_wq[0][(w[1] >> (31 - (q & 15))) & 1u];
+                    else return s_qw[(w[1 + ((q & 15) >> 2)] >> (8 * (q & 3))) & 0xFFu];
+                };
+                int nm = 0;
+                for (int p = tid; p < La; p += BLOCK) {
+                    const bool mis = mismatch(p);
+                    nm += mis;
+                    if (mis && (int)s_cov[p] >= o.clf_min_coverage) s_dec[atomicAdd(&s_nd, 1)] = (uint16_t)p;
                 }
-                const float nwin = (float)(hi - lo + 1);
-                x[16] = fdiv_rn(ssum, nwin);
-                x[17] = smin;
-                x[18] = fdiv_rn((float)nmis, (float)La);
-                int nloc = 0;
-                for (int q = max(p - 5, 0); q <= min(p + 5, La - 1); ++q)
-                    nloc += q != p && (s_aelem[q] & 3u) != s_cons[abegin + q];
-                x[19] = fdiv_rn((float)nloc, 10.0f);
-                x[20] = fdiv_rn((float)V, E);
-                x[21] = allGood ? 1.0f : 0.0f;
-                x[22] = (allGood || (s_support[col] > 0.90f && oc <= 2)) ? 1.0f : 0.0f;
-                x[23] = fdiv_rn(qsum, nwin);
-                const unsigned long long slot = atomicAdd(out.feat_count, 1ull);
-                if (slot >= out.feat_cap) { atomicOr(status, kStatusFeatOverflow); continue; }
-                float4* dst = reinterpret_cast<float4*>(out.feat + slot * kNumFeatures);
+                nm = __reduce_add_sync(0xffffffffu, nm);
+                if (lane == 0) s_red[warp] = nm;
+                __syncthreads();
+                int nmis = 0;
 #pragma unroll
-                for (int q = 0; q < kNumFeatures / 4; ++q) dst[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-                out.feat_read[slot] = a;
-                out.feat_meta[slot] = (uint32_t)p | (ob << 16) | (cb << 18);
+                for (int w = 0; w < NWARP; ++w) nmis += s_red[w];
+                const int maxCov = s_maxcov;
+                const float avgSup = s_avg, minSup = __int_as_float(s_min);
+                const int minCov = s_mincov;
+                const float Ec = o.estimated_coverage;
+                const int ndec = s_nd;
+                for (int i = tid; i < ndec; i += BLOCK) {
+                    const int p = s_dec[i];
+                    const uint32_t ce = s_cons[p + 16 * E];
+                    const uint32_t ob = ce >> 4, cb = ce & 3u;
+                    const float cov = (float)s_cov[p];
+                    const ushort4 c4 = s_cnt4[p];
+                    const int oc = ob == 0 ? c4.x : ob == 1 ? c4.y : ob == 2 ? c4.z : c4.w;
+                    const int cc = cb == 0 ? c4.x : cb == 1 ? c4.y : cb == 2 ? c4.z : c4.w;
+                    const float wsum = s_fw[p], wc = s_fw[mlen + p], wo = s_fw[2 * mlen + p];
+                    float x[kNumFeatures];
+                    x[0] = fdiv_rn((float)oc, cov);
+                    x[1] = fdiv_rn(wo, wsum);
+                    x[2] = fdiv_rn(wo, (float)oc);
+                    x[3] = fdiv_rn((float)cc, cov);
+                    x[4] = s_sup[p];
+                    x[5] = fdiv_rn(wc, (float)cc);
+                    x[6] = fdiv_rn(wsum, cov);
+                    x[7] = fdiv_rn(cov, Ec);
+                    x[8] = fdiv_rn(wsum, Ec);
+                    x[9] = avgSup;
+                    x[10] = minSup;
+                    x[11] = fdiv_rn((float)maxCov, Ec);
+                    x[12] = fdiv_rn((float)minCov, Ec);
+                    x[13] = anchor_weight(p);
+                    x[14] = fdiv_rn((float)min(p, La - 1 - p), (float)La);
+                    x[15] = fdiv_rn(fsub_rn(fsub_rn(wsum, wc), wo), wsum);
+                    const int lo = max(p - 3, 0), hi = min(p + 3, La - 1);
+                    float ssum = 0.0f, smin = s_sup[lo], qsum = 0.0f;
+                    for (int q = lo; q <= hi; ++q) {
+                        const float sv = s_sup[q];
+                        ssum = __fadd_rn(ssum, sv);
+                        if (sv < smin) smin = sv;
+                        qsum = __fadd_rn(qsum, anchor_weight(q));
+                    }
+                    const float nwin = (float)(hi - lo + 1);
+                    x[16] = fdiv_rn(ssum, nwin);
+                    x[17] = smin;
+                    x[18] = fdiv_rn((float)nmis, (float)La);
+                    int nloc = 0;
+                    for (int q = max(p - 5, 0); q <= min(p + 5, La - 1); ++q) nloc += q != p && mismatch(q);
+                    x[19] = fdiv_rn((float)nloc, 10.0f);
+                    x[20] = fdiv_rn((float)nalive, Ec);
+                    x[21] = allGood ? 1.0f : 0.0f;
+                    x[22] = (allGood || (s_sup[p] > 0.90f && oc <= 2)) ? 1.0f : 0.0f;
+                    x[23] = fdiv_rn(qsum, nwin);
+                    const unsigned long long slot = atomicAdd(out.feat_count, 1ull);
+                    if (slot >= out.feat_cap) { atomicOr(status, kStatusFeatOverflow); continue; }
+                    float4* dst = reinterpret_cast<float4*>(out.feat + slot * kNumFeatures);
+#pragma unroll
+                    for (int q = 0; q < kNumFeatures / 4; ++q) dst[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+                    out.feat_read[slot] = a;
+                    out.feat_meta[slot] = (uint32_t)p | (ob << 16) | (cb << 18);
+                }
             }
         }
+        if (!hq || !o.correct_candidates) return;
+
+        // ---- columns outside the anchor that its candidates' corrections
+        //      read: up to new_columns on each side, as far as rows reach ----
+        int mn = 0, mx = La;
+        for (int i = tid; i < nalive; i += BLOCK) {
+            int sft, L;
+            if (persistent) { const int k = (int)(s_ent[i + 1].w >> 4); sft = s_beg[k]; L = s_len[k]; }
+            else { const CandRec rc = recs[off + i]; sft = rc.shift; L = rc.len; }
+            mn = min(mn, sft);
+            mx = max(mx, sft + L);
+        }
+        mn = __reduce_min_sync(0xffffffffu, mn);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        __syncthreads();
+        if (lane == 0) { s_cnt[warp][0] = (uint32_t)mn; s_cnt[warp][1] = (uint32_t)mx; }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < NWARP; ++w) { mn = min(mn, (int)s_cnt[w][0]); mx = max(mx, (int)s_cnt[w][1]); }
+        const int left = min(-mn, 16 * E), right = min(mx - La, 16 * E);
+        for (int i = tid; i < left + right; i += BLOCK) s_col[i] = (int16_t)(i < left ? i - left : La + i - left);
+        if (tid == 0) s_nd = left + right;
+        outside = true;
+        __syncthreads();
     }
 
     // ---- candidate correction (getCorrectedCandidates, msa.cpp:457-522) ----
-    if (hq && o.correct_candidates) {
+    {
         const int ncc = o.new_columns;
-        for (int i = tid; i < V; i += BLOCK) {
+        for (int i = tid; i < nalive; i += BLOCK) {
             uint32_t id; int shift, L; bool fwd;
             if (persistent) {
-                const int k = s_alive[i];
+                const int k = (int)(s_ent[i + 1].w >> 4);
                 id = s_id[k]; shift = s_beg[k]; L = s_len[k]; fwd = s_fwd[k];
             } else {
                 const CandRec rc = recs[off + i];
                 id = rc.id; shift = rc.shift; L = rc.len; fwd = rc.orient == 1;
             }
-            const int qb = abegin + shift;
-            const int qe = qb + L;
-            if (!(abegin - ncc <= qb && qb <= abegin + ncc && qe <= aend + ncc)) continue;
+            if (!(-ncc <= shift && shift <= ncc && shift + L <= La + ncc)) continue;
             const unsigned long long slot = atomicAdd(out.corr_count, 1ull);
             if (slot >= out.corr_cap) { atomicOr(status, kStatusCorrOverflow); continue; }
             char* dst = out.corr_seq + slot * mlen;
             const uint32_t* row = r.seq + (size_t)id * sp;
+            const uint8_t* cons = s_cons + shift + 16 * E;
             int nd = 0;
             for (int p = 0; p < L; ++p) {
                 // forward orientation of the corrected candidate
-                const uint32_t cs = fwd ? s_cons[qb + p] : (s_cons[qb + L - 1 - p] ^ 3u);
+                const uint32_t cs = fwd ? cons[p] & 3u : (cons[L - 1 - p] & 3u) ^ 3u;
                 dst[p] = "ACGT"[cs];
                 nd += cs != base_at(row, p);
             }
@@ -1725,13 +1645,13 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
 // the hardware block scheduler hands out the anchors.
 template <int BLOCK, int QB, bool EMIT = false>
 __global__ void __launch_bounds__(BLOCK, (EMIT ? 768 : 1024) / BLOCK)
-k_msa(DevOptions o, DevReads r, uint32_t first, uint32_t count, int jb, const uint32_t* __restrict__ order,
+k_msa(DevOptions o, DevReads r, uint32_t first, uint32_t count, MsaGrid grid, const uint32_t* __restrict__ order,
       const uint32_t* __restrict__ cand_ids, const uint32_t* __restrict__ seg_off,
       const uint32_t* __restrict__ seg_cnt, const AlignRes* __restrict__ ares,
       CandRec* __restrict__ recs, MsaOut out, int* __restrict__ status) {
     if (blockIdx.x >= count) return;
     if (*status & kStatusCandOverflow) return;   // batch is repeated with a larger arena
-    msa_anchor<BLOCK, QB, EMIT>(o, r, first, order ? order[blockIdx.x] : blockIdx.x, jb, cand_ids, seg_off,
+    msa_anchor<BLOCK, QB, EMIT>(o, r, first, order ? order[blockIdx.x] : blockIdx.x, grid, cand_ids, seg_off,
                                 seg_cnt, ares, recs, out, status);
 }
 
@@ -1739,7 +1659,7 @@ k_msa(DevOptions o, DevReads r, uint32_t first, uint32_t count, int jb, const ui
 // queue (an atomic cursor over `order`) until the batch is done.
 template <int BLOCK, int QB, bool EMIT = false>
 __global__ void __launch_bounds__(BLOCK, (EMIT ? 768 : 1024) / BLOCK)
-k_msa_queue(DevOptions o, DevReads r, uint32_t first, uint32_t count, int jb, const uint32_t* __restrict__ order,
+k_msa_queue(DevOptions o, DevReads r, uint32_t first, uint32_t count, MsaGrid grid, const uint32_t* __restrict__ order,
             unsigned int* __restrict__ cursor, const uint32_t* __restrict__ cand_ids,
             const uint32_t* __restrict__ seg_off, const uint32_t* __restrict__ seg_cnt,
             const AlignRes* __restrict__ ares, CandRec* __restrict__ recs, MsaOut out,
@@ -1752,7 +1672,7 @@ k_msa_queue(DevOptions o, DevReads r, uint32_t first, uint32_t count, int jb, co
         __syncthreads();
         const uint32_t it = s_item;
         if (it >= count) return;
-        msa_anchor<BLOCK, QB, EMIT>(o, r, first, order ? order[it] : it, jb, cand_ids, seg_off, seg_cnt, ares,
+        msa_anchor<BLOCK, QB, EMIT>(o, r, first, order ? order[it] : it, grid, cand_ids, seg_off, seg_cnt, ares,
                                     recs, out, status);
     }
 }

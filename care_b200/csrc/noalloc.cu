@@ -222,23 +222,15 @@ extern "C" int care_b200_correct_range_noalloc(const care_b200_options* opt, con
     mo.seq = sequences;
     mo.corr_count = counters + 1;
     mo.corr_cap = 0;                     // no candidate corrections in this entry point
-    // widest possible MSA: La + 2*Lmax - 2*minoverlap(La), maximised over La
-    int maxcols = 1;
-    for (int la = 1; la <= r.max_len; ++la) {
-        const int lo = (int)((float)la * opt->min_overlap_ratio);
-        const int mo2 = lo > opt->min_overlap ? lo : opt->min_overlap;
-        const int c = la + 2 * r.max_len - 2 * (mo2 < r.max_len ? mo2 : r.max_len);
-        maxcols = c > maxcols ? c : maxcols;
-    }
-    const int jb = (maxcols + 127) / 128;
     const int qb = !o.use_quality ? 0 : o.quality_bits == 1 ? 1 : o.quality_bits == 2 ? 2 : 8;
-    const size_t msmem = msa_smem_bytes(r.max_len, r.seq_pitch, r.qual_pitch, qb, false, 128 * jb);
+    const MsaGrid mgrid = msa_grid(r.max_len, qb, 0, 0);
+    const size_t msmem = msa_smem_bytes(mgrid, r.max_len, false);
 #define LAUNCH_MSA(QB)                                                                                   \
     do {                                                                                                  \
         if (cudaFuncSetAttribute(k_msa<128, QB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem) \
             != cudaSuccess)                                                                               \
             return CARE_B200_ECUDA;                                                                       \
-        k_msa<128, QB><<<num_anchors, 128, msmem, st>>>(o, r, first_anchor, num_anchors, jb, nullptr,     \
+        k_msa<128, QB><<<num_anchors, 128, msmem, st>>>(o, r, first_anchor, num_anchors, mgrid, nullptr,     \
                                                         cand_ids, seg_off, seg_cnt, ares, recs, mo,       \
                                                         dstatus);                                         \
     } while (0)
@@ -252,6 +244,6 @@ extern "C" int care_b200_correct_range_noalloc(const care_b200_options* opt, con
     if (cudaMemcpyAsync(&hstatus, dstatus, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return CARE_B200_ECUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return CARE_B200_ECUDA;
     if (hstatus & kStatusTensorWait) return CARE_B200_ECUDA;
-    if (hstatus & (kStatusCandOverflow | kStatusColumns)) return CARE_B200_ELIMIT;
+    if (hstatus & kStatusCandOverflow) return CARE_B200_ELIMIT;
     return CARE_B200_OK;
 }

@@ -211,14 +211,14 @@ int care_b200_last_timing(const care_b200_ctx* ctx, float* total_ms, float* stag
  * stats[3] un-pruned 32-bit word compares of the alignment scans run (both
  * orientations, every scanned shift; a mirrored pair's shared scans count
  * once: the alignment stage's roofline work),
- * stats[4] bases added to MSA column sums (anchor and candidates, every
+ * stats[4] bases of the MSAs' rows (anchor and candidates, every
  * build including refinement rebuilds: the MSA stage's compute work),
  * stats[5] device batches the range was split into, stats[6] kernels of
  * this library launched (every batch and every arena-growth attempt),
  * stats[7] anchors whose candidate lists took the second, full-set pass,
  * stats[8] 32-bit word compares the alignment scans actually ran after their
  * early exits (counted only while care_b200_count_word_compares is on, else 0),
- * stats[9] bases added to MSA column sums by refinement rebuilds (the builds
+ * stats[9] bases of the MSAs' rows in refinement rebuilds (the builds
  * after an anchor's first; included in stats[4]), stats[10] anchors whose
  * MSA was rebuilt at least once (refineMSA, include/corrector.hpp:1307-1421). */
 int care_b200_last_stats(const care_b200_ctx* ctx, uint64_t* stats, int nstats);
