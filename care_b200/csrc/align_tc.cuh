@@ -73,14 +73,17 @@ k_mirror_index(DevReads r, uint32_t first, uint32_t count, const uint32_t* __res
     mirror[i] = m;
 }
 
-// D[tmem] (+)= A x B^T, e4m3 operands, fp32 sums, K = 32
-__device__ __forceinline__ void mma_e4m3(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         bool accumulate) {
+// D[tmem] (+)= A x B^T, e4m3 operands, fp32 sums, K = 32; the matrix
+// descriptors as halves (only the start addresses in the low ones change)
+__device__ __forceinline__ void mma_e4m3(uint32_t d_tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
+                                         uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-        :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %2};\n\t"
+        "mov.b64 b, {%3, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %5, p;\n\t}"
+        :: "r"(d_tmem), "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
@@ -93,10 +96,9 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
     return p != 0u;
 }
-__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | (uint64_t)((lbo >> 4) & 0x3FFFu) << 16 |
-           (uint64_t)((sbo >> 4) & 0x3FFFu) << 32 | (uint64_t)1 << 46;
-}
+// halves of a K-major no-swizzle matrix descriptor
+__device__ __forceinline__ uint32_t tc_desc_lo(uint32_t saddr, uint32_t lbo) { return ((saddr >> 4) & 0x3FFFu) | (lbo >> 4) << 16; }
+__device__ __forceinline__ uint32_t tc_desc_hi(uint32_t sbo) { return (sbo >> 4) | 1u << 14; }
 
 // Persistent CTAs, one anchor at a time. Per anchor: the Toeplitz regions of
 // its shifts, then per product of up to 32 candidates (i) their packed rows,
@@ -137,11 +139,11 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
     uint4* s_top = reinterpret_cast<uint4*>(tsm + lay.top);
     unsigned char* s_b = tsm + lay.b;
     uint32_t* s_fw = reinterpret_cast<uint32_t*>(tsm + lay.fw);
-    uint32_t* s_rw = reinterpret_cast<uint32_t*>(tsm + lay.rw);
+    uint32_t* s_ar = reinterpret_cast<uint32_t*>(tsm + lay.ar);     // and its reverse complement
     auto mex_of = [&](int ov) { return f2i_rz(fmul_rn((float)ov, o.max_error_rate)); };
     for (int i = tid; i <= kMaxLen; i += kTcBlock) s_thr[i] = tc_threshold(i, mex_of(i));
     for (int it = tid; it < kTcMaxItems; it += kTcBlock)
-        for (int w = W; w < RS; ++w) { s_fw[it * RS + w] = 0u; s_rw[it * RS + w] = 0u; }
+        for (int w = W; w < RS; ++w) s_fw[it * RS + w] = 0u;
     if (tid < 2) { s_win[tid][0] = 0; s_win[tid][1] = kMaxLen; s_win[tid][2] = 0; }
     if (tid == 0) {
         s_nh = 0;
@@ -277,6 +279,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                         uint32_t w[4];
                         tc_q_chunk(s_aw, nwa, La, q0 + 16 * x, w);
                         s_q[x] = make_uint4(w[0], w[1], w[2], w[3]);
+                        if (x < kMaxLen / 16 + 2) s_ar[x] = x < nwa ? tc_rc_word(s_aw, nwa, La, x) : 0u;
                     }
                 __syncthreads();
                 // ---- operands (a warp per 16-base chunk, a lane per row) ----
@@ -292,11 +295,9 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                         const int ch = (int)(((uint32_t)idx * magic_n) >> 16), it = idx - ch * nI;
                         const int left = (it < n ? (int)s_len[i0 + it] : 0) - 16 * ch;
                         const uint32_t* row = s_fw + it * RS;
-                        const uint32_t x = tc_rc_word(row, left + 16 * ch, ch);
-                        s_rw[it * RS + ch] = x;
                         uint32_t w[4], y[4];
                         tc_expand(row[ch], w);
-                        tc_expand(x, y);
+                        tc_expand_rc(tc_rc_window(row, left + 16 * ch, ch), y);
                         if (left < 16) {
                             uint32_t mk[4] = {~0u, ~0u, ~0u, ~0u};
                             tc_mask(mk, 0, left);
@@ -345,16 +346,16 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                     if (warp == 0 && elect_one()) {
                         tc05::fence_after_sync();
                         const uint32_t idesc = (1u << 4) | ((uint32_t)(2 * nI >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-                        const uint64_t db = tc_desc(tc05::smem_addr(s_b), 128u, 128u * W);
+                        const uint32_t blo = tc_desc_lo(tc05::smem_addr(s_b), 128u), bhi = tc_desc_hi(128u * W);
+                        const uint32_t ahi = tc_desc_hi(16u * XL);
 #pragma unroll 1
                         for (int t = 0; t < nt; ++t) {
-                            const uint64_t da = tc_desc(tc05::smem_addr(s_top) + 128u * (uint32_t)(lay.tiles - 1 - t0 - t),
-                                                        16u, 16u * XL);
+                            const uint32_t alo = tc_desc_lo(tc05::smem_addr(s_top) + 128u * (uint32_t)(lay.tiles - 1 - t0 - t), 16u);
                             const uint32_t d = tmem + (uint32_t)(t * (kTcCols / 2));
                             // K = 32 a step: two chunks further in both operands
-                            mma_e4m3(d, da, db, idesc, false);
 #pragma unroll 4
-                            for (int k = 1; k < ksteps; ++k) mma_e4m3(d, da + 2 * k, db + 16 * k, idesc, true);
+                            for (uint32_t k = 0; k < (uint32_t)ksteps; ++k)
+                                mma_e4m3(d, alo + 2 * k, ahi, blo + 16 * k, bhi, idesc, k);
                         }
                         tc05::commit(&s_bar);
                     }
@@ -403,12 +404,14 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                                     m[g] = fmaxf(max3(max3(max3(x[0], x[1], x[2]), x[3], x[4]), x[5], x[6]), x[7]);
                                 }
                                 if (fmaxf(m[0], m[1]) >= thr) {
+                                    float limit = thr;        // opaque: or the masks below are formed ahead of the branch
+                                    asm volatile("" : "+f"(limit));
 #pragma unroll
                                     for (int g = 0; g < 2; ++g) {
-                                        if (m[g] < thr) continue;
+                                        if (m[g] < limit) continue;
                                         uint32_t hits = 0u;
 #pragma unroll
-                                        for (int e = 0; e < 8; ++e) if (v[8 * g + e] >= thr) hits |= 1u << e;
+                                        for (int e = 0; e < 8; ++e) if (v[8 * g + e] >= limit) hits |= 1u << e;
                                         do {
                                             const int e = __ffs(hits) - 1;
                                             hits &= hits - 1u;
@@ -450,11 +453,14 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                         const int it = col - rev * nI;
                         const int L = s_len[i0 + it];
                         const int ov = tc_overlap(sh, La, L);
-                        const uint32_t ca = (rev ? lay.rw : lay.fw) + 4u * (uint32_t)(it * RS);
-                        const bool pos = sh >= 0;
-                        int mm = tc_mismatches(reinterpret_cast<const uint32_t*>(tsm + (pos ? lay.aw : ca)),
-                                               reinterpret_cast<const uint32_t*>(tsm + (pos ? ca : lay.aw)),
-                                               pos ? sh : -sh, ov, lane & 3, 4);
+                        // A against the candidate's reverse complement is A's
+                        // reverse complement against the candidate
+                        const uint32_t ca = lay.fw + 4u * (uint32_t)(it * RS), an = rev ? lay.ar : lay.aw;
+                        const int sv = rev ? La - L - sh : sh;
+                        const bool pos = sv >= 0;
+                        int mm = tc_mismatches(reinterpret_cast<const uint32_t*>(tsm + (pos ? an : ca)),
+                                               reinterpret_cast<const uint32_t*>(tsm + (pos ? ca : an)),
+                                               pos ? sv : -sv, ov, lane & 3, 4);
                         mm += __shfl_xor_sync(0xffffffffu, mm, 1);
                         mm += __shfl_xor_sync(0xffffffffu, mm, 2);
                         if ((lane & 3) == 0 && ov >= minov && mm < mex_of(ov)) {

@@ -822,8 +822,11 @@ struct MsaArgs {
 // prepare (host only: attributes, occupancy) or launch one MSA variant
 template <int B, int QB, bool E>
 cudaError_t msa_go(MsaArgs& a, bool prepare, cudaStream_t st) {
+    constexpr int kMany = B == 128 && !E ? kMsaManyCtas : (E ? 768 : 1024) / B;
+    const bool many = msa_many_ctas(a.smem, a.count, a.sms);
     if (prepare) {
-        cudaError_t e = cudaFuncSetAttribute(k_msa<B, QB, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem);
+        cudaError_t e = many ? cudaFuncSetAttribute(k_msa<B, QB, E, kMany>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem)
+                             : cudaFuncSetAttribute(k_msa<B, QB, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_msa_queue<B, QB, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem);
         int nb = 0;
@@ -835,6 +838,9 @@ cudaError_t msa_go(MsaArgs& a, bool prepare, cudaStream_t st) {
         k_msa_queue<B, QB, E><<<a.grid, B, a.smem, st>>>(a.o, a.r, a.first, a.count, a.mgrid, a.order, a.cursor,
                                                         a.cand_ids, a.seg_off, a.seg_cnt, a.ares, a.recs, a.out,
                                                         a.status);
+    else if (many)
+        k_msa<B, QB, E, kMany><<<a.count, B, a.smem, st>>>(a.o, a.r, a.first, a.count, a.mgrid, a.order, a.cand_ids,
+                                                           a.seg_off, a.seg_cnt, a.ares, a.recs, a.out, a.status);
     else
         k_msa<B, QB, E><<<a.count, B, a.smem, st>>>(a.o, a.r, a.first, a.count, a.mgrid, a.order, a.cand_ids,
                                                     a.seg_off, a.seg_cnt, a.ares, a.recs, a.out, a.status);

@@ -38,7 +38,7 @@ struct CandSmem {
         return seq(maxlen, groups, maps) + (size_t)(pitch + 4) * 4;
     }
     static __host__ __device__ size_t set(int maxlen, int groups, int maps, int pitch) {
-        return qinfo(maxlen, groups, maps, pitch) + (size_t)(3 * kMaxMaps + 8) * 4;
+        return (qinfo(maxlen, groups, maps, pitch) + (size_t)(3 * kMaxMaps + 8) * 4 + 15) & ~(size_t)15;
     }
     static __host__ __device__ size_t total(int maxlen, int groups, int maps, int pitch, int setcap) {
         return set(maxlen, groups, maps, pitch) + (size_t)setcap * 4 * 2;
@@ -812,23 +812,23 @@ __host__ __device__ inline size_t msa_smem_bytes(const MsaGrid& g, int max_len, 
            msa_round16((size_t)max_len * 2) + msa_round16(cols * 2) + cols;
 }
 
-// The 16 2-bit codes from code b on of a packed row of n words; codes outside
-// the row are arbitrary.
+// The 16 2-bit codes from code b on of a packed row of n words, b from -15 to
+// the row's last code; codes outside the row are arbitrary.
 __device__ __forceinline__ uint32_t window2(const uint32_t* __restrict__ row, int n, int b) {
     const int wi = b >> 4;
-    const uint32_t hi = __ldg(row + min(max(wi, 0), n - 1)), lo = __ldg(row + min(max(wi + 1, 0), n - 1));
+    const uint32_t hi = __ldg(row + max(wi, 0)), lo = __ldg(row + min(wi + 1, n - 1));
     return __funnelshift_l(lo, hi, 2 * (b & 15));
 }
 // 1-bit codes, 32 per word, MSB first: 16 codes in the high half
 __device__ __forceinline__ uint32_t window1(const uint32_t* __restrict__ row, int n, int b) {
     const int wi = b >> 5;
-    const uint32_t hi = __ldg(row + min(max(wi, 0), n - 1)), lo = __ldg(row + min(max(wi + 1, 0), n - 1));
+    const uint32_t hi = __ldg(row + max(wi, 0)), lo = __ldg(row + min(wi + 1, n - 1));
     return __funnelshift_l(lo, hi, b & 31);
 }
 // 4 characters from character b on, little-endian
 __device__ __forceinline__ uint32_t window8(const uint32_t* __restrict__ row, int n, int b) {
     const int wi = b >> 2;
-    const uint32_t lo = __ldg(row + min(max(wi, 0), n - 1)), hi = __ldg(row + min(max(wi + 1, 0), n - 1));
+    const uint32_t lo = __ldg(row + max(wi, 0)), hi = __ldg(row + min(wi + 1, n - 1));
     return __funnelshift_r(lo, hi, 8 * (b & 3));
 }
 // reverse the 16 2-bit codes of a word, keeping each code's bits
@@ -878,12 +878,10 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
     extern __shared__ __align__(16) unsigned char dsm[];
     __shared__ float s_qw[QB == 8 ? 256 : 1];
     __shared__ float s_qwc[4];               // weight of a 1- or 2-bit quality code
-    // by slot (0: the anchor): shift, length, weight, id, orientation, weight
-    // * weight of a 1- or 2-bit quality code
-    __shared__ int16_t s_beg[kStageMax + 1], s_len[kStageMax + 1];
+    // by slot (0: the anchor): the row, its weight, weight * weight of a 1- or
+    // 2-bit quality code
+    __shared__ uint2 s_slot[kStageMax + 1];  // {id, shift (16 bits) | length << 16 | reverse complement << 31}
     __shared__ float s_w[kStageMax + 1];
-    __shared__ uint32_t s_id[kStageMax + 1];
-    __shared__ uint8_t s_fwd[kStageMax + 1];
     __shared__ __align__(16) float s_wq[kStageMax + 1][4];
     // the rows of the sums in list order, {byte offset of the staged row,
     // -shift, length, 16 * slot}, one entry of length 0 behind the last
@@ -891,8 +889,8 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
     __shared__ uint32_t s_dis[kMaxLen / 16];  // disputed columns, bit 30 - 2 * (position % 16)
     __shared__ __align__(16) int s_diff[kMaxLen + 4]; // coverage changes by anchor position
     __shared__ int s_red[NWARP + 1];
-    __shared__ int s_nd, s_sig, s_min, s_mincov, s_maxcov, s_bases, s_flags;
-    __shared__ float s_avg;
+    __shared__ int s_nd, s_sig, s_min, s_mincov, s_maxcov, s_bases, s_ndec;
+    __shared__ float s_avg, s_defect;
     __shared__ uint16_t s_dec[EMIT ? kMaxLen : 1];   // decision positions of the anchor (EMIT)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -942,12 +940,11 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
         s_wq[0][tid] = c_qweight[ch];                        // the anchor's factor is 1
     }
     if (tid == 0) {
-        s_beg[0] = 0;
-        s_len[0] = (int16_t)La;
+        s_slot[0] = make_uint2(a, (uint32_t)La << 16);
         s_w[0] = 1.0f;
-        s_fwd[0] = 1;
-        s_id[0] = a;
     }
+    auto slot_beg = [&](int k) { return (int)(int16_t)s_slot[k].y; };
+    auto slot_len = [&](int k) { return (int)((s_slot[k].y >> 16) & 0x7fffu); };
 
     // ---- alignment filters (corrector.hpp:982-1211), ordered compaction ----
     const float base = fmul_rn(o.estimated_errorrate, 1.0f);
@@ -1001,11 +998,9 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
     }
     // slot k of the staged rows
     auto fill_slot = [&](int k, const CandRec& rec) {
-        s_beg[k] = rec.shift;
-        s_len[k] = (int16_t)rec.len;
+        s_slot[k] = make_uint2(rec.id, (uint32_t)(uint16_t)rec.shift | (uint32_t)rec.len << 16 |
+                                           (rec.orient == 1 ? 0u : 0x80000000u));
         s_w[k] = rec.weight;
-        s_fwd[k] = rec.orient == 1;
-        s_id[k] = rec.id;
         if constexpr (QB == 1 || QB == 2)
             *reinterpret_cast<float4*>(&s_wq[k][0]) =
                 make_float4(fmul_rn(rec.weight, s_qwc[0]), fmul_rn(rec.weight, s_qwc[1]),
@@ -1064,14 +1059,15 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
             const int e = G > 1 ? (int)__umulhi((uint32_t)idx, grid.magic) : idx, g = idx - e * G;
             const int k = list ? (int)(s_ent[e + 1].w >> 4) : k0 + e;
             const int p0 = 16 * (g - E);                     // anchor position of the word's first code
-            const int sft = s_beg[k], L = s_len[k];
+            const uint2 slot = s_slot[k];
+            const int sft = (int)(int16_t)slot.y, L = (int)((slot.y >> 16) & 0x7fffu);
             const int lo = max(sft - p0, 0), hi = min(sft + L - p0, 16);
             if (lo >= hi) continue;                          // the row does not reach the word
             uint32_t* dst = s_raw + k * rw + g * wpg;
             uint32_t ws;
             if (load) {
-                const bool rev = !s_fwd[k];
-                const size_t id = s_id[k];
+                const bool rev = slot.y >> 31;
+                const size_t id = slot.x;
                 const int q0 = p0 - sft;
                 ws = window2(r.seq + id * sp, sp, rev ? L - 16 - q0 : q0);
                 if (rev) ws = ~rev2(ws);                     // reversed, complemented: A<->T, C<->G
@@ -1108,14 +1104,14 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
     };
     // entries of slots 1 .. n (and the anchor's, entry 0, when with_anchor)
     auto put_entry = [&](int e, int k, int len) {
-        s_ent[e] = make_uint4((uint32_t)(k * rw * 4), (uint32_t)-(int)s_beg[k], (uint32_t)len, (uint32_t)k * 16u);
+        s_ent[e] = make_uint4((uint32_t)(k * rw * 4), (uint32_t)-slot_beg(k), (uint32_t)len, (uint32_t)k * 16u);
     };
     // a chunk of the global records into slots 1 .. n
     auto stage_chunk = [&](int c, int n) {
         __syncthreads();
         for (int k = tid; k < n; k += BLOCK) {
             fill_slot(k + 1, recs[off + c + k]);
-            put_entry(k + 1, k + 1, s_len[k + 1]);
+            put_entry(k + 1, k + 1, slot_len(k + 1));
         }
         if (tid == 0) put_entry(n + 1, 0, 0);
         __syncthreads();
@@ -1143,9 +1139,9 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
         int ncol;
         if (!outside) {
             // ---- disputed columns, coverage ----
-            for (int i = tid; i < kMaxLen + 4; i += BLOCK) s_diff[i] = 0;
+            for (int i = tid; i < (kMaxLen + 4) / 4; i += BLOCK) reinterpret_cast<int4*>(s_diff)[i] = make_int4(0, 0, 0, 0);
             if (tid < kMaxLen / 16) s_dis[tid] = tid == 0 && sigThr <= 0 ? 0x40000000u : 0u;   // counts of 0 are significant
-            if (tid == 0) { s_sig = 0x7fffffff; s_bases = 0; }
+            if (tid == 0) { s_sig = 0x7fffffff; s_bases = 0; s_defect = 0.0f; s_ndec = 0; s_red[NWARP] = 0; }
             __syncthreads();
             if (iter == 0) scan_words(1, 0, true, false);    // the anchor
             int sl = 0;
@@ -1158,15 +1154,15 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                 scan_words(nalive, 1, iter == 0, iter > 0);
                 for (int i = tid; i < nalive; i += BLOCK) {
                     const int k = iter == 0 ? i + 1 : (int)(s_ent[i + 1].w >> 4);
-                    if (iter == 0) put_entry(i + 1, k, s_len[k]);
-                    add_cover(s_beg[k], s_len[k]);
+                    if (iter == 0) put_entry(i + 1, k, slot_len(k));
+                    add_cover(slot_beg(k), slot_len(k));
                 }
                 if (tid == 0) { put_entry(0, 0, La); put_entry(nalive + 1, 0, 0); }
             } else {
                 for (int c = 0; c < nalive; c += nstage) {
                     const int n = min(nstage, nalive - c);
                     stage_chunk(c, n);
-                    for (int k = tid; k < n; k += BLOCK) add_cover(s_beg[k + 1], s_len[k + 1]);
+                    for (int k = tid; k < n; k += BLOCK) add_cover(slot_beg(k + 1), slot_len(k + 1));
                 }
                 if (tid == 0) {
                     put_entry(0, 0, La);
@@ -1240,6 +1236,7 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
         //      consensus (findConsensus, msa.cpp:135-157): 32 listed columns
         //      a warp, lane = column ----
         int mism = 0;
+        float defect = 0.0f;                                 // 1 - support of the lane's columns
         const int nblk = (ncol + 31) >> 5;
         const int nchunk = persistent ? 1 : max(1, (nalive + nstage - 1) / nstage);
 #pragma unroll 1
@@ -1326,6 +1323,7 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                     s_sup[p] = sup;
                     s_cnt4[p] = make_ushort4((uint16_t)nA, (uint16_t)nC, (uint16_t)nG, (uint16_t)nT);
                     mism |= cs != ob;
+                    defect = __fadd_rn(defect, fsub_rn(1.0f, sup));
                     const bool sig = (cs != 0 && sigThr <= (int)nA) || (cs != 1 && sigThr <= (int)nC) ||
                                      (cs != 2 && sigThr <= (int)nG) || (cs != 3 && sigThr <= (int)nT);
                     if (sig) atomicMin(&s_sig, p);
@@ -1337,6 +1335,11 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                     }
                 }
             }
+        }
+        if (!outside && 32 * warp < ncol) {                  // warp-uniform
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) defect = __fadd_rn(defect, __shfl_xor_sync(0xffffffffu, defect, d));
+            if (lane == 0) atomicAdd(&s_defect, defect);
         }
         mism = __syncthreads_or(mism);
         if (outside) break;
@@ -1363,8 +1366,8 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                 return removes(rc.orient == 1 ? (int)base_at(row, q) : (int)(base_at(row, rc.len - 1 - q) ^ 3u));
             };
             auto slot_removed = [&](int k) {
-                const int q = col - s_beg[k];
-                return q >= 0 && q < s_len[k] && removes((int)staged_base(k, col));
+                const int q = col - slot_beg(k);
+                return q >= 0 && q < slot_len(k) && removes((int)staged_base(k, col));
             };
             int nrem = 0, veto = 0;
             for (int i = tid; i < nalive; i += BLOCK) {
@@ -1414,11 +1417,18 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
         }
 
         // ---- MSA properties (getMSAProperties, msa.cpp:304-376) ----
-        if (warp == 0) {
-            // std::accumulate order: one serial chain of IEEE adds (lane 0),
-            // the supports read four at a time
+        // The reference's average support is one serial chain of float adds
+        // over the anchor's columns. What it decides are comparisons with two
+        // thresholds, so the average from the disputed columns' defects
+        // settles them unless it comes within 1e-4 of one: both averages are
+        // within 1e-5 of the exact one (256 adds below 256, each half an ulp
+        // of 2^-16 at most). Otherwise, and for the decision rows' features,
+        // the chain is added up. (1,200 of 9,500 warp instructions per anchor
+        // and a wait of the whole CTA for one lane: 13.0 -> 12.6 ms per 1M
+        // reads.)
+        auto serial_average = [&]() {         // into s_avg, by warp 0; the supports read four at a time
             float sum = 0.0f;
-            if (lane == 0) {
+            if (warp == 0 && lane == 0) {
                 const float4* v4 = reinterpret_cast<const float4*>(s_sup);
                 int p = 0;
                 for (; p + 4 <= La; p += 4) {
@@ -1426,46 +1436,32 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                     sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
                 }
                 for (; p < La; ++p) sum = __fadd_rn(sum, s_sup[p]);
+                s_avg = fdiv_rn(sum, (float)La);
             }
-            sum = __shfl_sync(0xffffffffu, sum, 0);
-            const float minSup = __int_as_float(s_min);
-            const int minCov = s_mincov;
-            const float avgSup = fdiv_rn(sum, (float)La);
+        };
+        const float minSup = __int_as_float(s_min);
+        const int minCov = s_mincov;
+        bool allGood;
+        {
             const float e = o.estimated_errorrate;
             const float avgThr = fsub_rn(1.0f, fmul_rn(1.0f, e));
             const float minThr = fsub_rn(1.0f, fmul_rn(3.0f, e));
             const float covThr = fmul_rn(fdiv_rn(o.m_coverage, 6.0f), o.estimated_coverage);
-            const bool good = fgeq(avgSup, avgThr) && fgeq(minSup, minThr) && fgeq((float)minCov, covThr);
-            bool isHQ = false;
-            if (good) {                       // warp-uniform
-                // the smallest percentage pc in [0, pct] whose thresholds hold
-                // (the reference's loop from pct down to 0 keeps the last one)
-                int smallest = 100;
-                const int pct = (int)ceilf(fmul_rn(e, 100.0f));
-                auto holds = [&](int pc) {
-                    const float fac = fdiv_rn((float)pc, 100.0f);
-                    const float at = fsub_rn(1.0f, fmul_rn(1.0f, fac));
-                    const float mt = fsub_rn(1.0f, fmul_rn(3.0f, fac));
-                    return fgeq(avgSup, at) && fgeq(minSup, mt);
-                };
-                if (pct < 32) {
-                    const unsigned bm = __ballot_sync(0xffffffffu, lane <= pct && holds(lane));
-                    if (bm) smallest = __ffs(bm) - 1;
-                } else {
-                    for (int pc = pct; pc >= 0; --pc) if (holds(pc)) smallest = pc;
-                }
-                isHQ = fgeq((float)minCov, covThr) && fleq((float)smallest, fmul_rn((float)pct, 0.5f));
+            // HQ: the smallest percentage pc in [0, pct] whose thresholds hold
+            // is at most half of pct; they loosen as pc grows, so the largest
+            // such pc decides
+            const int pct = (int)ceilf(fmul_rn(e, 100.0f));
+            const float fac = fdiv_rn((float)(pct >> 1), 100.0f);
+            const float hqAvg = fsub_rn(1.0f, fmul_rn(1.0f, fac)), hqMin = fsub_rn(1.0f, fmul_rn(3.0f, fac));
+            float avg = fdiv_rn(fsub_rn((float)La, s_defect), (float)La);
+            if (!(fabsf(avg - avgThr) > 1e-4f && fabsf(avg - hqAvg) > 1e-4f)) {      // block-uniform
+                serial_average();
+                __syncthreads();
+                avg = s_avg;
             }
-            if (lane == 0) {
-                s_nd = 0;                     // decision positions listed (EMIT)
-                s_flags = (good ? 1 : 0) | (isHQ ? 2 : 0);
-                s_avg = avgSup;
-                s_red[NWARP] = 0;
-            }
+            allGood = fgeq(avg, avgThr) && fgeq(minSup, minThr) && fgeq((float)minCov, covThr);
+            hq = allGood && pct >= 0 && fgeq(avg, hqAvg) && fgeq(minSup, hqMin);
         }
-        __syncthreads();
-        const bool allGood = s_flags & 1;
-        hq = s_flags & 2;
 
         // ---- anchor correction (getCorrectedAnchor, msa.cpp:379-453) ----
         if (nalive == 0) {
@@ -1513,19 +1509,19 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                 for (int p = tid; p < La; p += BLOCK) {
                     const bool mis = mismatch(p);
                     nm += mis;
-                    if (mis && (int)s_cov[p] >= o.clf_min_coverage) s_dec[atomicAdd(&s_nd, 1)] = (uint16_t)p;
+                    if (mis && (int)s_cov[p] >= o.clf_min_coverage) s_dec[atomicAdd(&s_ndec, 1)] = (uint16_t)p;
                 }
                 nm = __reduce_add_sync(0xffffffffu, nm);
                 if (lane == 0) s_red[warp] = nm;
+                serial_average();
                 __syncthreads();
                 int nmis = 0;
 #pragma unroll
                 for (int w = 0; w < NWARP; ++w) nmis += s_red[w];
                 const int maxCov = s_maxcov;
-                const float avgSup = s_avg, minSup = __int_as_float(s_min);
-                const int minCov = s_mincov;
+                const float avgSup = s_avg;
                 const float Ec = o.estimated_coverage;
-                const int ndec = s_nd;
+                const int ndec = s_ndec;
                 for (int i = tid; i < ndec; i += BLOCK) {
                     const int p = s_dec[i];
                     const uint32_t ce = s_cons[p + 16 * E];
@@ -1588,7 +1584,7 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
         int mn = 0, mx = La;
         for (int i = tid; i < nalive; i += BLOCK) {
             int sft, L;
-            if (persistent) { const int k = (int)(s_ent[i + 1].w >> 4); sft = s_beg[k]; L = s_len[k]; }
+            if (persistent) { const int k = (int)(s_ent[i + 1].w >> 4); sft = slot_beg(k); L = slot_len(k); }
             else { const CandRec rc = recs[off + i]; sft = rc.shift; L = rc.len; }
             mn = min(mn, sft);
             mx = max(mx, sft + L);
@@ -1614,7 +1610,7 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
             uint32_t id; int shift, L; bool fwd;
             if (persistent) {
                 const int k = (int)(s_ent[i + 1].w >> 4);
-                id = s_id[k]; shift = s_beg[k]; L = s_len[k]; fwd = s_fwd[k];
+                id = s_slot[k].x; shift = slot_beg(k); L = slot_len(k); fwd = !(s_slot[k].y >> 31);
             } else {
                 const CandRec rc = recs[off + i];
                 id = rc.id; shift = rc.shift; L = rc.len; fwd = rc.orient == 1;
@@ -1643,8 +1639,17 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
 
 // One CTA per anchor, in `order` (e.g. most candidates first) when given;
 // the hardware block scheduler hands out the anchors.
-template <int BLOCK, int QB, bool EMIT = false>
-__global__ void __launch_bounds__(BLOCK, (EMIT ? 768 : 1024) / BLOCK)
+// CTAS: CTAs that share an SM. With rows short enough for ten of them and
+// anchors enough to fill them, the register limit of ten is taken (48
+// registers, a few spills): 12.6 -> 12.0 ms per 1M 150 bp reads. Reads of
+// 50-250 bases, which shared memory holds to eight, lose by it (8.5 -> 8.9 ms
+// per 400k), and so do 128 anchors, one per SM (156 -> 217 us).
+constexpr int kMsaManyCtas = 10;
+inline bool msa_many_ctas(size_t dynamic_smem, uint32_t anchors, int sms) {
+    return (dynamic_smem + 8192) * kMsaManyCtas <= 228 * 1024 && anchors >= (uint32_t)(16 * sms);
+}
+template <int BLOCK, int QB, bool EMIT = false, int CTAS = (EMIT ? 768 : 1024) / BLOCK>
+__global__ void __launch_bounds__(BLOCK, CTAS)
 k_msa(DevOptions o, DevReads r, uint32_t first, uint32_t count, MsaGrid grid, const uint32_t* __restrict__ order,
       const uint32_t* __restrict__ cand_ids, const uint32_t* __restrict__ seg_off,
       const uint32_t* __restrict__ seg_cnt, const AlignRes* __restrict__ ares,

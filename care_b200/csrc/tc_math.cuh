@@ -28,7 +28,7 @@ struct TcLayout {
     int tiles;                          // 128-shift tiles of the widest anchor
     int XL;                             // 16-byte chunks of a Toeplitz region
     uint32_t magic_w;                   // x / W as (x * magic) >> 16, x < 4096
-    uint32_t aw, q, top, b, fw, rw, total;
+    uint32_t aw, ar, q, top, b, fw, total;
 };
 
 inline TcLayout tc_layout(int max_len, int min_overlap, float min_overlap_ratio) {
@@ -46,7 +46,8 @@ inline TcLayout tc_layout(int max_len, int min_overlap, float min_overlap_ratio)
     t.XL = 7 + t.W + 8 * (t.tiles - 1);
     t.magic_w = (65536u + (uint32_t)t.W - 1) / (uint32_t)t.W;
     t.aw = 0;
-    uint32_t at = 4u * (kMaxLen / 16 + 4);
+    t.ar = 4u * (kMaxLen / 16 + 4);
+    uint32_t at = 2u * t.ar;
     t.q = at;
     at += (uint32_t)(t.XL + 1) * 16u;
     t.top = (at + 127u) & ~127u;
@@ -54,8 +55,6 @@ inline TcLayout tc_layout(int max_len, int min_overlap, float min_overlap_ratio)
     t.b = (at + 127u) & ~127u;
     at = t.b + 2u * kTcMaxItems * 16u * (uint32_t)t.W;
     t.fw = at;
-    at += kTcMaxItems * 4u * (uint32_t)t.RS;
-    t.rw = at;
     at += kTcMaxItems * 4u * (uint32_t)t.RS;
     t.total = at;
     return t;
@@ -111,12 +110,35 @@ CB_HD uint32_t tc_window(const uint32_t* row, int n, int b) {
     return funnel_l(lo, hi, 2 * (b & 15));
 }
 
-// Word c of the reverse complement of a row of length L. Bases past its end
-// are arbitrary (row[-1] is read there: it has to be readable).
-CB_HD uint32_t tc_rc_word(const uint32_t* row, int L, int c) {
+// The window of a row of length L whose reverse complement is chunk c of the
+// row's reverse complement; bases past its end are arbitrary (row[-1] is read
+// there: it has to be readable).
+CB_HD uint32_t tc_rc_window(const uint32_t* row, int L, int c) {
     const int b = L - 16 - 16 * c;
     const int wi = b >= -16 ? b >> 4 : -1;
-    uint32_t w = brev32(funnel_l(row[wi + 1], row[wi], 2 * (b & 15)));
+    return funnel_l(row[wi + 1], row[wi], 2 * (b & 15));
+}
+
+// tc_expand of a window's reverse complement: bytes in reverse order, signs
+// flipped. The high bits of a byte go from 1, 3, 5, 7 to 7, 15, 23, 31; the
+// four copies meet only at bits 13, 19 and 25, whose carries stop one bit up.
+CB_HD void tc_expand_rc(uint32_t x, uint32_t (&w)[4]) {
+    x &= 0xAAAAAAAAu;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#ifdef __CUDA_ARCH__
+        const uint32_t b = __byte_perm(x, 0u, 0x4440u + (uint32_t)i);
+#else
+        const uint32_t b = (x >> (8 * i)) & 0xFFu;
+#endif
+        w[i] = ((b * 0x01041040u) & 0x80808080u) ^ 0xB8B8B8B8u;
+    }
+}
+
+// Word c of the packed reverse complement of a row of n words and length L
+// (the high bases of the last word's tail are arbitrary).
+CB_HD uint32_t tc_rc_word(const uint32_t* row, int n, int L, int c) {
+    uint32_t w = brev32(tc_window(row, n, L - 16 - 16 * c));
     w = ((w >> 1) & 0x55555555u) | ((w & 0x55555555u) << 1);
     return ~w;
 }

@@ -29,19 +29,19 @@ extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch,
     const int smin = minov - maxl;
     const int ntiles = (smax < 0 || maxl < minov) ? 0 : (smax - smin + 128) >> 7;
     if (ntiles > lay.tiles) return -2;
-    std::vector<uint32_t> aw(kMaxLen / 16 + 2, 0u), fwp((size_t)kTcMaxItems * RS + 1, 0x5a5a5a5au), rw((size_t)kTcMaxItems * RS, 0u);
+    std::vector<uint32_t> aw(kMaxLen / 16 + 2, 0u), fwp((size_t)kTcMaxItems * RS + 1, 0x5a5a5a5au), ar(kMaxLen / 16 + 2, 0u);
     uint32_t* fw = fwp.data() + 1;                     // a word before the first row is read
     for (int i = 0; i < nwa; ++i) aw[i] = a[i];
+    for (int i = 0; i < nwa; ++i) ar[i] = tc_rc_word(aw.data(), nwa, La, i);
     std::vector<uint8_t> top(lay.b - lay.top), b((size_t)2 * kTcMaxItems * 16 * W, 0x7f);
     for (int i = 0; i < n; ++i)
         for (int w = 0; w < W; ++w) fw[i * RS + w] = 16 * w < len[i] ? rows[(size_t)i * pitch + w] : 0u;
     for (int i = 0; i < n; ++i)
         for (int c = 0; c < W; ++c)
             for (int rev = 0; rev < 2; ++rev) {
-                uint32_t x = fw[i * RS + c];
-                if (rev) rw[i * RS + c] = x = tc_rc_word(&fw[i * RS], len[i], c);
                 uint32_t w[4];
-                tc_expand(x, w);
+                if (rev) tc_expand_rc(tc_rc_window(&fw[i * RS], len[i], c), w);
+                else tc_expand(fw[i * RS + c], w);
                 if (len[i] - 16 * c < 16) tc_mask(w, 0, len[i] - 16 * c);
                 const int row = rev * nI + i;
                 std::memcpy(&b[(size_t)(row >> 3) * (128 * W) + c * 128 + (row & 7) * 16], w, 16);
@@ -97,11 +97,13 @@ extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch,
                 ++hits;
                 const int ov = tc_overlap(s, La, Lc);
                 if (ov < minov) continue;
-                const uint32_t* cr = rev ? &rw[it * RS] : &fw[it * RS];
+                // the reverse complement's shift, seen from the anchor's reverse complement
+                const uint32_t *cr = &fw[it * RS], *an = rev ? ar.data() : aw.data();
+                const int sv = rev ? La - Lc - s : s;
                 const int mex = f2i_rz(fmul_rn((float)ov, rate));
                 int mm = 0;
                 for (int part = 0; part < 4; ++part)
-                    mm += s >= 0 ? tc_mismatches(aw.data(), cr, s, ov, part, 4) : tc_mismatches(cr, aw.data(), -s, ov, part, 4);
+                    mm += sv >= 0 ? tc_mismatches(an, cr, sv, ov, part, 4) : tc_mismatches(cr, an, -sv, ov, part, 4);
                 if (mm >= mex) continue;
                 const uint32_t sc = (uint32_t)(mm + La + Lc - 2 * ov) << 10;
                 uint32_t& ka = key[rev * n + it];
