@@ -46,31 +46,37 @@ inline bool tc_applies(float max_error_rate, int min_overlap, float min_overlap_
            min_overlap_ratio >= 0.0f && min_overlap_ratio <= 1.0f;
 }
 
-// Mirror of each pair of the batch (see k_pair_mirror): kMirrorSkip when its
-// mirror answers it (a > c), its mirror's index when it leads, kMirrorSingle
-// when it has none.
+// Mirror of each pair of the batch (see k_pair_mirror): its mirror's index
+// when it leads (a < c), kMirrorSkip when its mirror answers it; the caller
+// has set every entry to kMirrorSingle. Only leaders search (the mirror of a
+// pair exists exactly when the leader finds it) and write both entries, and
+// the pair flag of the mirror's result, whose search through global memory
+// would hold up a whole CTA of the alignment. With a search per pair and the
+// flags searched there, the alignment of 1.3M reads at 50x took 29.8 ms.
 static __global__ void __launch_bounds__(256)
-k_mirror_index(DevReads r, uint32_t first, uint32_t count, const uint32_t* __restrict__ cand_ids,
+k_mirror_index(DevReads r, int paired_end, uint32_t first, uint32_t count, const uint32_t* __restrict__ cand_ids,
                const uint32_t* __restrict__ cand_anchor, const uint32_t* __restrict__ seg_off,
                const uint32_t* __restrict__ seg_cnt, const unsigned long long* __restrict__ total_ptr,
-               unsigned long long arena_cap, const int* __restrict__ status, uint32_t* __restrict__ mirror) {
+               unsigned long long arena_cap, const int* __restrict__ status, uint32_t* __restrict__ mirror,
+               AlignRes* __restrict__ out) {
     if (*status & kStatusCandOverflow) return;
     const unsigned long long total = *total_ptr;
     if (total > arena_cap) return;
     const unsigned long long i = (unsigned long long)blockIdx.x * 256 + threadIdx.x;
     if (i >= total) return;
     const uint32_t a = first + cand_anchor[i], c = cand_ids[i];
-    uint32_t m = kMirrorSingle;
-    if (c - first < count && r.len[a] == r.len[c]) {
-        const uint32_t ci = c - first, off = seg_off[ci], cnt = seg_cnt[ci];
-        uint32_t lo = 0, hi = cnt;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (cand_ids[off + mid] < a) lo = mid + 1; else hi = mid;
-        }
-        if (lo < cnt && cand_ids[off + lo] == a) m = a < c ? off + lo : kMirrorSkip;
+    if (c <= a || c - first >= count || r.len[a] != r.len[c]) return;
+    const uint32_t ci = c - first, off = seg_off[ci], cnt = seg_cnt[ci];
+    uint32_t lo = 0, hi = cnt;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (cand_ids[off + mid] < a) lo = mid + 1; else hi = mid;
     }
-    mirror[i] = m;
+    if (lo < cnt && cand_ids[off + lo] == a) {
+        mirror[i] = off + lo;
+        mirror[off + lo] = kMirrorSkip;
+        out[off + lo].paired = paired_end ? mate_flag(cand_ids, seg_off, seg_cnt, ci, a) : 0;
+    }
 }
 
 // D[tmem] (+)= A x B^T, e4m3 operands, fp32 sums, K = 32; the matrix
@@ -106,8 +112,7 @@ __device__ __forceinline__ uint32_t tc_desc_hi(uint32_t sbo) { return (sbo >> 4)
 // 128-shift tile, (iii) every sum against its shift's threshold (a warp reads
 // its 32 shifts of all columns), the possible ones listed, (iv) their exact
 // counts and a minimum per column, (v) the orientation, the pair flag and the
-// AlignRes. The next anchor's segment, ids and lengths load meanwhile, and one
-// warp writes an anchor's results while the others begin the next.
+// AlignRes. The next anchor's segment, ids and lengths load meanwhile.
 // mirror (may be null): k_mirror_index's array; a leading pair also writes
 // its mirror's result. splits: parts that an anchor's candidates are handed
 // out in (tc_splits).
@@ -127,7 +132,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
     __shared__ uint32_t s_idb[2][kTcWindow], s_mirb[2][kTcWindow], s_mateb[2][kTcMate];
     __shared__ uint16_t s_lenb[2][kTcWindow];
     __shared__ uint8_t s_pib[2][kTcWindow];
-    __shared__ uint32_t s_hit[kTcHits];
+    __shared__ uint32_t s_hit[kTcHits];                // column | (shift + 512) << 16
     __shared__ uint32_t s_key[3][kTcMaxItems];         // best of (A, C), (A, rc C), (C, A)
     __shared__ __align__(16) float s_kl[kTcMaxItems];  // kappa * length
     if (*status & kStatusCandOverflow) return;         // arena entries past the overflow are unwritten
@@ -416,7 +421,8 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                                             const int e = __ffs(hits) - 1;
                                             hits &= hits - 1u;
                                             const int p = atomicAdd(&s_nh, 1);
-                                            if (p < kTcHits) s_hit[p] = (uint32_t)(q + 8 * g + e) << 10 | (uint32_t)(s + 512);
+                                            if (p < kTcHits)
+                                                s_hit[p] = (uint32_t)(q + 8 * g + e) | (uint32_t)(s + 512) << 16;
                                         } while (hits);
                                     }
                                 }
@@ -446,8 +452,8 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                             if (col >= n) col += nI - n;
                         } else {
                             const uint32_t hv = s_hit[k];
-                            col = (int)(hv >> 10);
-                            sh = (int)(hv & 1023u) - 512;
+                            col = (int)(hv & 0xFFFFu);
+                            sh = (int)(hv >> 16) - 512;
                         }
                         const int rev = col >= nI;
                         const int it = col - rev * nI;
@@ -471,40 +477,44 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                     }
                 }
                 __syncthreads();
-                // ---- orientation and results, by one warp; the others
-                //      go on (nothing read here is written before the next
-                //      barrier) ----
-                if (warp == 1 && lane < n) {
-                    const int it = lane;
-                    const int L = s_len[i0 + it];
-                    const uint32_t id = s_id[i0 + it], m = s_mir[i0 + it];
-                    const ShdResult rc = tc_result(s_key[1][it], La, L);
-                    // the pair itself, then its mirror (equal lengths: the
-                    // same reverse-complement alignment)
-#pragma unroll 1
-                    for (int side = 0; side < (m != kMirrorSingle ? 2 : 1); ++side) {
+                // ---- orientation and results. With mirrors eight items a
+                //      warp, lanes 0-7 the pair, lanes 8-15 its mirror (equal
+                //      lengths: the same reverse-complement alignment; its
+                //      pair flag is written already); else by one warp, while
+                //      the others go on (four warps: 0.7 ms more per 1M reads).
+                //      Nothing read here is written before the next two
+                //      barriers ----
+                {
+                    const int it = mirror ? 8 * warp + (lane & 7) : lane;
+                    const int side = mirror ? lane >> 3 : warp == 1 ? 0 : 2;
+                    if (it < n && side < 2 && (side == 0 || s_mir[i0 + it] != kMirrorSingle)) {
+                        const int L = s_len[i0 + it];
+                        const ShdResult rc = tc_result(s_key[1][it], La, L);
                         const ShdResult fw = tc_result(s_key[side ? 2 : 0][it], La, L);
                         const int orr = choose_orientation(fw, rc, La, o.min_overlap_ratio, o.min_overlap, ler);
                         const ShdResult& b = orr == 2 ? rc : fw;
-                        AlignRes res;
-                        res.shift = (int16_t)b.shift;
-                        res.overlap = (int16_t)b.overlap;
-                        res.nops = (int16_t)b.nops;
-                        res.orient = (uint8_t)orr;
-                        res.paired = 0;
-                        if (o.paired_end && orr != 3) {
-                            const bool here = side == 0 && mcnt <= (uint32_t)kTcMate;
-                            const uint32_t mo = side ? (id - first) ^ 1u : ai ^ 1u;
-                            const uint32_t* list = here ? s_mate : cand_ids + seg_off[mo];
-                            const uint32_t len = here ? mcnt : seg_cnt[mo], target = (side ? a : id) ^ 1u;
-                            uint32_t l = 0, h = len;
-                            while (l < h) {
-                                const uint32_t mid = (l + h) >> 1;
-                                if (list[mid] < target) l = mid + 1; else h = mid;
+                        AlignRes* dst = out + (side ? (size_t)s_mir[i0 + it] : (size_t)off + w0 + s_pi[i0 + it]);
+                        dst->shift = (int16_t)b.shift;
+                        dst->overlap = (int16_t)b.overlap;
+                        dst->nops = (int16_t)b.nops;
+                        dst->orient = (uint8_t)orr;
+                        if (side == 0) {
+                            uint8_t paired = 0;
+                            if (o.paired_end && orr != 3) {
+                                const uint32_t target = s_id[i0 + it] ^ 1u;
+                                if (mcnt <= (uint32_t)kTcMate) {
+                                    uint32_t l = 0, h = mcnt;
+                                    while (l < h) {
+                                        const uint32_t mid = (l + h) >> 1;
+                                        if (s_mate[mid] < target) l = mid + 1; else h = mid;
+                                    }
+                                    paired = l < mcnt && s_mate[l] == target;
+                                } else {
+                                    paired = mate_flag(cand_ids, seg_off, seg_cnt, ai, s_id[i0 + it]);
+                                }
                             }
-                            res.paired = l < len && list[l] == target;
+                            dst->paired = paired;
                         }
-                        out[side ? m : off + w0 + s_pi[i0 + it]] = res;
                     }
                 }
             }

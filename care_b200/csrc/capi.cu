@@ -1031,10 +1031,12 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
             EQ(mark(1), "event");
             if (tc) {
                 if (tu.pair_mirror) {
+                    EQ(cudaMemsetAsync(ctx->d_pair_work.p, 0xff, cap * 4, st), "memset");     // kMirrorSingle
                     k_mirror_index<<<(unsigned)((cap + 255) / 256), 256, 0, st>>>(
-                        r, first, count, ctx->d_cand_ids.as<uint32_t>(), ctx->d_cand_anchor.as<uint32_t>(),
-                        ctx->d_seg_off.as<uint32_t>(), ctx->d_seg_cnt.as<uint32_t>(), counters, cap, status,
-                        ctx->d_pair_work.as<uint32_t>());
+                        r, o.paired_end, first, count, ctx->d_cand_ids.as<uint32_t>(),
+                        ctx->d_cand_anchor.as<uint32_t>(), ctx->d_seg_off.as<uint32_t>(),
+                        ctx->d_seg_cnt.as<uint32_t>(), counters, cap, status, ctx->d_pair_work.as<uint32_t>(),
+                        ctx->d_ares.as<AlignRes>());
                     EQ(cudaGetLastError(), "k_mirror_index");
                     ++launches;
                 }
