@@ -27,12 +27,13 @@
 // of one M = 128 tile: 4.3 KB instead of 20 KB at K = 160, and the copy that
 // would write them.
 //
-// Bound: instruction issue (13K warp instructions per anchor of 47 candidates;
-// the products take a tenth of the tensor pipe, 46 cycles per 128 x 48 x 32
-// step, the same as with a stored Toeplitz matrix). Measured against the
-// thread scan (k_align, its pair mirroring included): 1M 150 bp paired-end
-// reads at 30x 15.9 ms (18.8), 400k reads of 50-250 bases 19.6 ms (34.1),
-// 300k 100 bp reads 4.1 ms (5.6), 128 anchors 27 us (58).
+// Bound: instruction issue and barriers (57 % issue active, 13K warp
+// instructions per anchor of 47 candidates; the products take a tenth of the
+// tensor pipe, 46 cycles per 128 x 64 x 32 step, the same as with a stored
+// Toeplitz matrix). Measured against the thread scan (k_align) and its pair
+// mirroring: 1M 150 bp paired-end reads at 30x 14.3 ms (18.8), 1.3M at 50x
+// 24.3 ms (36.3), 400k reads of 50-250 bases 11.8 ms with mirrors, 18.0 ms
+// without (34.1), 300k 100 bp reads 3.1 and 4.1 ms (5.6), 128 anchors 28 us (58).
 #pragma once
 #include "kernels.cuh"
 #include "tc05.cuh"
@@ -46,9 +47,11 @@ inline bool tc_applies(float max_error_rate, int min_overlap, float min_overlap_
            min_overlap_ratio >= 0.0f && min_overlap_ratio <= 1.0f;
 }
 
-// Mirror of each pair of the batch (see k_pair_mirror): its mirror's index
-// when it leads (a < c), kMirrorSkip when its mirror answers it; the caller
-// has set every entry to kMirrorSingle. Only leaders search (the mirror of a
+// Mirror of each pair of the batch: its mirror's index when it leads,
+// kMirrorSkip when its mirror answers it; the caller has set every entry to
+// kMirrorSingle. The shorter read leads (the smaller id of equal lengths): its
+// minimum overlap is the smaller one, so its shifts include the mirror's.
+// Only leaders search (the mirror of a
 // pair exists exactly when the leader finds it) and write both entries, and
 // the pair flag of the mirror's result, whose search through global memory
 // would hold up a whole CTA of the alignment. With a search per pair and the
@@ -65,7 +68,9 @@ k_mirror_index(DevReads r, int paired_end, uint32_t first, uint32_t count, const
     const unsigned long long i = (unsigned long long)blockIdx.x * 256 + threadIdx.x;
     if (i >= total) return;
     const uint32_t a = first + cand_anchor[i], c = cand_ids[i];
-    if (c <= a || c - first >= count || r.len[a] != r.len[c]) return;
+    if (c - first >= count) return;
+    const int La = r.len[a], Lc = r.len[c];
+    if (La > Lc || (La == Lc && c <= a)) return;
     const uint32_t ci = c - first, off = seg_off[ci], cnt = seg_cnt[ci];
     uint32_t lo = 0, hi = cnt;
     while (lo < hi) {
@@ -133,7 +138,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
     __shared__ uint16_t s_lenb[2][kTcWindow];
     __shared__ uint8_t s_pib[2][kTcWindow];
     __shared__ uint32_t s_hit[kTcHits];                // column | (shift + 512) << 16
-    __shared__ uint32_t s_key[3][kTcMaxItems];         // best of (A, C), (A, rc C), (C, A)
+    __shared__ uint32_t s_key[4][kTcMaxItems];         // best of (A, C), (A, rc C), (C, A), (C, rc A)
     __shared__ __align__(16) float s_kl[kTcMaxItems];  // kappa * length
     if (*status & kStatusCandOverflow) return;         // arena entries past the overflow are unwritten
     if (*total_ptr > arena_cap) return;
@@ -145,6 +150,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
     unsigned char* s_b = tsm + lay.b;
     uint32_t* s_fw = reinterpret_cast<uint32_t*>(tsm + lay.fw);
     uint32_t* s_ar = reinterpret_cast<uint32_t*>(tsm + lay.ar);     // and its reverse complement
+    auto minov_of = [&](int L) { return max(o.min_overlap, f2i_rz(fmul_rn((float)L, o.min_overlap_ratio))); };
     auto mex_of = [&](int ov) { return f2i_rz(fmul_rn((float)ov, o.max_error_rate)); };
     for (int i = tid; i <= kMaxLen; i += kTcBlock) s_thr[i] = tc_threshold(i, mex_of(i));
     for (int it = tid; it < kTcMaxItems; it += kTcBlock)
@@ -193,8 +199,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
     }
     while (unit < units) {
         const uint32_t a = first + ai;
-        const int lo = __float2int_rz(__fmul_rn((float)La, o.min_overlap_ratio));
-        const int minov = o.min_overlap > lo ? o.min_overlap : lo;
+        const int minov = minov_of(La);
         const int smax = La - minov;
         const int nwa = (La + 15) >> 4;
         const int q0 = smax - 127 - 128 * (lay.tiles - 1);    // base of the first operand chunk
@@ -289,7 +294,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                 __syncthreads();
                 // ---- operands (a warp per 16-base chunk, a lane per row) ----
                 if (tid < kTcMaxItems) {
-                    s_key[0][tid] = s_key[1][tid] = s_key[2][tid] = 0xFFFFFFFFu;
+                    s_key[0][tid] = s_key[1][tid] = s_key[2][tid] = s_key[3][tid] = 0xFFFFFFFFu;
                     s_kl[tid] = tid < n ? kappa * (float)s_len[i0 + tid] : 0.0f;
                 }
                 if (tid == 0) s_nh = 0;
@@ -472,14 +477,13 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                         if ((lane & 3) == 0 && ov >= minov && mm < mex_of(ov)) {
                             const uint32_t sc = (uint32_t)(mm + La + L - 2 * ov) << 10;
                             atomicMin(&s_key[rev][it], sc | tc_rank(sh));
-                            if (!rev) atomicMin(&s_key[2][it], sc | tc_rank(-sh));
+                            if (mirror && ov >= minov_of(L)) atomicMin(&s_key[2 + rev][it], sc | tc_rank(tc_mirror_shift(sh, rev, La, L)));
                         }
                     }
                 }
                 __syncthreads();
                 // ---- orientation and results. With mirrors eight items a
-                //      warp, lanes 0-7 the pair, lanes 8-15 its mirror (equal
-                //      lengths: the same reverse-complement alignment; its
+                //      warp, lanes 0-7 the pair, lanes 8-15 its mirror (its
                 //      pair flag is written already); else by one warp, while
                 //      the others go on (four warps: 0.7 ms more per 1M reads).
                 //      Nothing read here is written before the next two
@@ -489,9 +493,10 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                     const int side = mirror ? lane >> 3 : warp == 1 ? 0 : 2;
                     if (it < n && side < 2 && (side == 0 || s_mir[i0 + it] != kMirrorSingle)) {
                         const int L = s_len[i0 + it];
-                        const ShdResult rc = tc_result(s_key[1][it], La, L);
-                        const ShdResult fw = tc_result(s_key[side ? 2 : 0][it], La, L);
-                        const int orr = choose_orientation(fw, rc, La, o.min_overlap_ratio, o.min_overlap, ler);
+                        const int L1 = side ? L : La, L2 = side ? La : L;
+                        const ShdResult fw = tc_result(s_key[2 * side][it], L1, L2);
+                        const ShdResult rc = tc_result(s_key[2 * side + 1][it], L1, L2);
+                        const int orr = choose_orientation(fw, rc, L1, o.min_overlap_ratio, o.min_overlap, ler);
                         const ShdResult& b = orr == 2 ? rc : fw;
                         AlignRes* dst = out + (side ? (size_t)s_mir[i0 + it] : (size_t)off + w0 + s_pi[i0 + it]);
                         dst->shift = (int16_t)b.shift;

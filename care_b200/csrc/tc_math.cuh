@@ -174,6 +174,10 @@ CB_HD int tc_mismatches(const uint32_t* x, const uint32_t* y, int t, int ov, int
 CB_HD uint32_t tc_rank(int s) { return (uint32_t)(s >= 0 ? s : 512 - s); }
 CB_HD int tc_rank_shift(uint32_t r) { return r < 512u ? (int)r : 512 - (int)r; }
 
+// The shift of the mirrored pair (C as anchor, A or its reverse complement as
+// candidate) that compares the same bases as (A, C) or (A, rc C) at s.
+CB_HD int tc_mirror_shift(int s, int rev, int La, int Lc) { return rev ? s - (La - Lc) : -s; }
+
 // ShdResult of a scan from its best key (all ones: no shift).
 CB_HD ShdResult tc_result(uint32_t key, int La, int Lc) {
     ShdResult res;

@@ -11,9 +11,10 @@ using namespace careb200;
 
 static float e4m3(uint8_t b) { return b == 0x38 ? 1.0f : b == 0xB8 ? -1.0f : b == 0 ? 0.0f : 1e30f; }
 
-// rows: n candidates of `pitch` words. out: 16 ints per candidate -- score,
-// overlap, shift, nops, valid of (A, C), of (A, rc C) and of (C, A), then the
-// orientation. per_column: the threshold form of mixed lengths. Returns the
+// rows: n candidates of `pitch` words. out: 22 ints per candidate -- score,
+// overlap, shift, nops, valid of (A, C), of (A, rc C), of (C, A) and of (C, rc
+// A) (for a candidate not shorter than the anchor), then the orientations of
+// (A, C) and (C, A). per_column: the threshold form of mixed lengths. Returns the
 // possible shifts listed, -1 on a byte no operand holds, -2 on an index past
 // a buffer.
 extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch, const int* len, int n, int max_len,
@@ -63,7 +64,7 @@ extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch,
         }
     for (int idx = 0; idx < kTcMaxItems * W; ++idx)
         if ((int)(((uint32_t)idx * lay.magic_w) >> 16) != idx / W) return -2;
-    std::vector<uint32_t> key((size_t)3 * n, 0xFFFFFFFFu);
+    std::vector<uint32_t> key((size_t)4 * n, 0xFFFFFFFFu);
     const float kappa = 1.0f - 2.0f * rate;
     int hits = 0;
     const int K = 32 * ((maxl + 31) / 32);
@@ -108,20 +109,24 @@ extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch,
                 const uint32_t sc = (uint32_t)(mm + La + Lc - 2 * ov) << 10;
                 uint32_t& ka = key[rev * n + it];
                 ka = ka < (sc | tc_rank(s)) ? ka : sc | tc_rank(s);
-                uint32_t& kc = key[2 * n + it];
-                if (!rev) kc = kc < (sc | tc_rank(-s)) ? kc : sc | tc_rank(-s);
+                const int lc = f2i_rz(fmul_rn((float)Lc, ratio));
+                if (ov < (min_overlap > lc ? min_overlap : lc)) continue;
+                uint32_t& kc = key[(2 + rev) * n + it];
+                const uint32_t m = sc | tc_rank(tc_mirror_shift(s, rev, La, Lc));
+                kc = kc < m ? kc : m;
             }
         }
     for (int it = 0; it < n; ++it) {
-        const ShdResult f = tc_result(key[it], La, len[it]), r = tc_result(key[n + it], La, len[it]),
-                        g = tc_result(key[2 * n + it], len[it], La);
-        const ShdResult* rs[3] = {&f, &r, &g};
-        int* o = out + 16 * it;
-        for (int k = 0; k < 3; ++k) {
-            o[5 * k] = rs[k]->score; o[5 * k + 1] = rs[k]->overlap; o[5 * k + 2] = rs[k]->shift;
-            o[5 * k + 3] = rs[k]->nops; o[5 * k + 4] = rs[k]->valid;
+        const int L = len[it];
+        const ShdResult rs[4] = {tc_result(key[it], La, L), tc_result(key[n + it], La, L),
+                                 tc_result(key[2 * n + it], L, La), tc_result(key[3 * n + it], L, La)};
+        int* o = out + 22 * it;
+        for (int k = 0; k < 4; ++k) {
+            o[5 * k] = rs[k].score; o[5 * k + 1] = rs[k].overlap; o[5 * k + 2] = rs[k].shift;
+            o[5 * k + 3] = rs[k].nops; o[5 * k + 4] = rs[k].valid;
         }
-        o[15] = choose_orientation(f, r, La, ratio, min_overlap, fmul_rn(est, 4.0f));
+        o[20] = choose_orientation(rs[0], rs[1], La, ratio, min_overlap, fmul_rn(est, 4.0f));
+        o[21] = choose_orientation(rs[2], rs[3], L, ratio, min_overlap, fmul_rn(est, 4.0f));
     }
     return hits;
 }

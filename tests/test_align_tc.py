@@ -61,7 +61,7 @@ def _oracle_one(a, c, mo, rate, ratio):
 FIXED = [16, 17, 31, 32, 33, 64, 100, 150, 151, 255, 256]
 
 
-@pytest.mark.parametrize("seed", range(60))
+@pytest.mark.parametrize("seed", range(90))
 def test_operands_and_results_match_the_oracle(lib, seed):
     rng = random.Random(300 + seed)
     uniform = seed % 2 == 0
@@ -84,14 +84,14 @@ def test_operands_and_results_match_the_oracle(lib, seed):
     max_len = max([La] + lens)
     pitch = (max_len + 15) // 16
     rows = np.stack([_enc(c, pitch) for c in cands])
-    rows[:, -1] |= np.uint32(0x5)        # storage past a read's end need not be zero
+    rows[:, -1] |= np.uint32(0x1)        # storage past a read's end need not be zero
     rows = np.where((np.arange(pitch)[None, :] * 16 + 16 <= np.array(lens)[:, None]) |
                     (np.array(lens)[:, None] % 16 == 0), np.stack([_enc(c, pitch) for c in cands]), rows)
     ln = np.array(lens, np.int32)
     aw = _enc(a, 17)
     got = []
     for per_column in ([0, 1] if uniform else [1]):
-        out = np.zeros((n, 16), np.int32)
+        out = np.zeros((n, 22), np.int32)
         rc = lib.hd_tc(aw.ctypes.data_as(ctypes.c_void_p), La, rows.ctypes.data_as(ctypes.c_void_p), pitch,
                        ln.ctypes.data_as(ctypes.c_void_p), n, max_len, mo, ctypes.c_float(rate), ctypes.c_float(ratio),
                        ctypes.c_float(0.06), per_column, out.ctypes.data_as(ctypes.c_void_p))
@@ -101,18 +101,26 @@ def test_operands_and_results_match_the_oracle(lib, seed):
         assert np.array_equal(got[0], out)
     minov = max(mo, int(np.float32(La) * np.float32(ratio)))
     for i, c in enumerate(cands):
-        f, r = _oracle_one(a, c, mo, rate, ratio), _oracle_one(a, _rc(c), mo, rate, ratio)
-        want = _oracle.lib().co_orientation(ctypes.byref(f), ctypes.byref(r), La, lens[i], ctypes.c_float(ratio), mo,
-                                            ctypes.c_float(0.06))
         o = got[0][i]
-        assert o[15] == want
-        if want in (1, 2):
-            b = f if want == 1 else r
-            assert list(o[5 * (want - 1):5 * want]) == [b.score, b.overlap, b.shift, b.nops, b.valid]
-        if lens[i] == La and La >= minov:                # the mirrored direction and both orientations
-            m = _oracle_one(c, a, mo, rate, ratio)
-            for k, x in enumerate((f, r, m)):
-                assert list(o[5 * k:5 * k + 5]) == [x.score, x.overlap, x.shift, x.nops, x.valid]
+
+        def check(x, y, at, orient):
+            """(x, y) with x as anchor: results from o[at], the orientation."""
+            f, r = _oracle_one(x, y, mo, rate, ratio), _oracle_one(x, _rc(y), mo, rate, ratio)
+            want = _oracle.lib().co_orientation(ctypes.byref(f), ctypes.byref(r), len(x), len(y), ctypes.c_float(ratio),
+                                                mo, ctypes.c_float(0.06))
+            assert orient == want
+            if want in (1, 2):
+                b = f if want == 1 else r
+                at += 5 * (want - 1)
+                assert list(o[at:at + 5]) == [b.score, b.overlap, b.shift, b.nops, b.valid]
+            return f, r
+
+        f, r = check(a, c, 0, o[20])
+        if lens[i] >= La:                                # the mirrored pair
+            m, mr = check(c, a, 10, o[21])
+            if lens[i] == La and La >= minov:            # every alignment in full
+                for k, x in enumerate((f, r, m, mr)):
+                    assert list(o[5 * k:5 * k + 5]) == [x.score, x.overlap, x.shift, x.nops, x.valid]
 
 
 def test_random_pairs_rarely_stay_possible(lib):
@@ -123,7 +131,7 @@ def test_random_pairs_rarely_stay_possible(lib):
     a = _rand(rng, L)
     rows = np.stack([_enc(_rand(rng, L), 10) for _ in range(n)])
     ln = np.full(n, L, np.int32)
-    out = np.zeros((n, 16), np.int32)
+    out = np.zeros((n, 22), np.int32)
     hits = lib.hd_tc(_enc(a, 17).ctypes.data_as(ctypes.c_void_p), L, rows.ctypes.data_as(ctypes.c_void_p), 10,
                      ln.ctypes.data_as(ctypes.c_void_p), n, L, 30, ctypes.c_float(0.2), ctypes.c_float(0.3),
                      ctypes.c_float(0.06), 0, out.ctypes.data_as(ctypes.c_void_p))

@@ -44,7 +44,7 @@ def _run(seqs, lengths, count_words, ranges, tuning=None, **opts):
                 assert (st["word_compares_run"] > 0) == count_words
             o = np.lexsort((r.cand_anchor_ids, r.cand_read_ids))
             out.append([r.status, r.num_edits, r.sequences, r.cand_read_ids[o], r.cand_anchor_ids[o], r.cand_shifts[o],
-                        r.cand_use_edits[o], r.cand_sequences[o], np.array([st["pairs"], st["word_compares"]])])
+                        r.cand_use_edits[o], r.cand_sequences[o], np.array([st["pairs"], 0 if (tuning or {}).get("pair_mirror") else st["word_compares"]])])
     return out
 
 
@@ -56,12 +56,13 @@ def _same(seqs, lengths, ranges, **kw):
     return a
 
 
+@pytest.mark.parametrize("mirror", [0, 1])           # 1: pairs of any lengths answered with their mirrors
 @pytest.mark.parametrize("lo,hi", [(100, 100), (50, 250), (33, 64), (256, 256)])
-def test_long_candidate_lists(lo, hi):
+def test_long_candidate_lists(lo, hi, mirror):
     genome = np.random.default_rng(lo).integers(0, 4, 4 * (lo + hi))
     seqs, lengths = _reads(1, 1500, lo, hi, genome)
     res = _same(seqs, lengths, [(0, 1500), (3, 1), (17, 333)], kmerlength=16, num_maps=8, estimated_coverage=400.0,
-                correct_candidates=1, min_overlap=30)
+                correct_candidates=1, min_overlap=30, tuning={"pair_mirror": mirror})
     assert res[0][8][0] > 1500 * 128                     # several windows of 128
 
 
@@ -88,5 +89,6 @@ def test_short_tandem_repeats(unit):
 def test_option_edges(rate, overlap, ratio):
     genome = np.random.default_rng(9).integers(0, 4, 3000)
     seqs, lengths = _reads(4, 800, 60, 200, genome)
-    _same(seqs, lengths, [(0, 800)], kmerlength=16, num_maps=16, estimated_coverage=80.0, max_error_rate=rate,
-          min_overlap=overlap, min_overlap_ratio=ratio)
+    for mirror in (0, 1):
+        _same(seqs, lengths, [(0, 800)], kmerlength=16, num_maps=16, estimated_coverage=80.0, max_error_rate=rate,
+              min_overlap=overlap, min_overlap_ratio=ratio, tuning={"pair_mirror": mirror})
