@@ -23,6 +23,13 @@ CB_HD uint32_t funnel_l(uint32_t lo, uint32_t hi, int r) {   // high word of (hi
     return (uint32_t)(((((unsigned long long)hi) << 32) | lo) << (r & 31) >> 32);
 #endif
 }
+CB_HD uint32_t funnel_r(uint32_t lo, uint32_t hi, int r) {   // low word of (hi:lo) >> r
+#ifdef __CUDA_ARCH__
+    return __funnelshift_r(lo, hi, r);
+#else
+    return (uint32_t)(((((unsigned long long)hi) << 32) | lo) >> (r & 31));
+#endif
+}
 CB_HD int popc32(uint32_t x) {
 #ifdef __CUDA_ARCH__
     return __popc(x);
@@ -197,6 +204,41 @@ CB_HD unsigned long long kmer_at(const uint32_t* s, int k, int pos) {
 // 2-bit code of base p of a packed row.
 CB_HD uint32_t base_at(const uint32_t* s, int p) {
     return (s[p >> 4] >> (30 - 2 * (p & 15))) & 3u;
+}
+
+// The codes a staged word of the MSA takes from a row, part `part` of `codes`
+// codes each, when the word's first code lies q0 (-15 .. length - 1) after the
+// row's first one: the first code read of a row of `span` codes that is read
+// forward or, turned, from its end.
+CB_HD int staged_start(bool rev, int span, int q0, int codes, int part) {
+    const int q = q0 + codes * part;
+    return rev ? span - codes - q : q;
+}
+
+// Windows of a row of n words; codes outside the row are arbitrary, words
+// outside it are never read. Row: const uint32_t*.
+// The 16 2-bit codes from code b on, b from -15 to the row's last code.
+template <class Row>
+CB_HD uint32_t window2(Row row, int n, int b) {
+    const int wi = b >> 4;
+    const uint32_t hi = ldg32(row + max(wi, 0)), lo = ldg32(row + min(wi + 1, n - 1));
+    return funnel_l(lo, hi, 2 * (b & 15));
+}
+// 1-bit codes, 32 per word, MSB first: 16 codes in the high half, b as above
+template <class Row>
+CB_HD uint32_t window1(Row row, int n, int b) {
+    const int wi = b >> 5;
+    const uint32_t hi = ldg32(row + max(wi, 0)), lo = ldg32(row + min(wi + 1, n - 1));
+    return funnel_l(lo, hi, b & 31);
+}
+// 4 characters from character b on, little-endian. The four parts of a grid
+// word whose ends alone reach the row start up to 15 characters before it and
+// up to 12 after its last one, so both words are held to both ends.
+template <class Row>
+CB_HD uint32_t window8(Row row, int n, int b) {
+    const int wi = b >> 2;
+    const uint32_t lo = ldg32(row + min(max(wi, 0), n - 1)), hi = ldg32(row + min(max(wi + 1, 0), n - 1));
+    return funnel_r(lo, hi, 8 * (b & 3));
 }
 
 // Compress the even bits (0,2,...,30) of x into the low 16 bits, order kept.

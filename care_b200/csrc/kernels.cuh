@@ -838,25 +838,6 @@ __host__ __device__ inline size_t msa_smem_bytes(const MsaGrid& g, int max_len, 
            msa_round16((size_t)max_len * 2) + msa_round16(cols * 2) + cols;
 }
 
-// The 16 2-bit codes from code b on of a packed row of n words, b from -15 to
-// the row's last code; codes outside the row are arbitrary.
-__device__ __forceinline__ uint32_t window2(const uint32_t* __restrict__ row, int n, int b) {
-    const int wi = b >> 4;
-    const uint32_t hi = __ldg(row + max(wi, 0)), lo = __ldg(row + min(wi + 1, n - 1));
-    return __funnelshift_l(lo, hi, 2 * (b & 15));
-}
-// 1-bit codes, 32 per word, MSB first: 16 codes in the high half
-__device__ __forceinline__ uint32_t window1(const uint32_t* __restrict__ row, int n, int b) {
-    const int wi = b >> 5;
-    const uint32_t hi = __ldg(row + max(wi, 0)), lo = __ldg(row + min(wi + 1, n - 1));
-    return __funnelshift_l(lo, hi, b & 31);
-}
-// 4 characters from character b on, little-endian
-__device__ __forceinline__ uint32_t window8(const uint32_t* __restrict__ row, int n, int b) {
-    const int wi = b >> 2;
-    const uint32_t lo = __ldg(row + max(wi, 0)), hi = __ldg(row + min(wi + 1, n - 1));
-    return __funnelshift_r(lo, hi, 8 * (b & 3));
-}
 // reverse the 16 2-bit codes of a word, keeping each code's bits
 __device__ __forceinline__ uint32_t rev2(uint32_t w) {
     w = __brev(w);
@@ -1095,22 +1076,22 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
                 const bool rev = slot.y >> 31;
                 const size_t id = slot.x;
                 const int q0 = p0 - sft;
-                ws = window2(r.seq + id * sp, sp, rev ? L - 16 - q0 : q0);
+                ws = window2(r.seq + id * sp, sp, staged_start(rev, L, q0, 16, 0));
                 if (rev) ws = ~rev2(ws);                     // reversed, complemented: A<->T, C<->G
                 if constexpr (QB == 2) {
-                    uint32_t wq = window2(r.qual + id * qp, qp, rev ? mlen - 16 - q0 : q0);
+                    uint32_t wq = window2(r.qual + id * qp, qp, staged_start(rev, mlen, q0, 16, 0));
                     if (rev) wq = rev2(wq);
                     *reinterpret_cast<uint2*>(dst) = make_uint2(ws, wq);
                 } else {
                     dst[0] = ws;
                     if constexpr (QB == 1) {
-                        uint32_t wq = window1(r.qual + id * qp, qp, rev ? mlen - 16 - q0 : q0);
+                        uint32_t wq = window1(r.qual + id * qp, qp, staged_start(rev, mlen, q0, 16, 0));
                         if (rev) wq = __brev(wq) << 16;
                         dst[1] = wq;
                     } else if constexpr (QB == 8) {
 #pragma unroll
                         for (int h = 0; h < 4; ++h) {
-                            uint32_t wq = window8(r.qual + id * qp, qp, rev ? mlen - 4 - q0 - 4 * h : q0 + 4 * h);
+                            uint32_t wq = window8(r.qual + id * qp, qp, staged_start(rev, mlen, q0, 4, h));
                             if (rev) wq = __byte_perm(wq, 0u, 0x0123);
                             dst[1 + h] = wq;
                         }
