@@ -42,6 +42,8 @@
 
 namespace careb200 {
 
+constexpr uint32_t kTcWaitLimit = 1u << 22;
+
 // Whether the tensor-core alignment takes these options.
 inline bool tc_applies(float max_error_rate, int min_overlap, float min_overlap_ratio) {
     return max_error_rate >= 0.0f && max_error_rate <= kTcMaxErrorRate && min_overlap >= 1 &&
@@ -121,13 +123,15 @@ __device__ __forceinline__ uint32_t tc_desc_hi(uint32_t sbo) { return (sbo >> 4)
 // AlignRes. The next anchor's segment, ids and lengths load meanwhile.
 // mirror (may be null): k_mirror_index's array; a leading pair also writes
 // its mirror's result. splits: parts that an anchor's candidates are handed
-// out in (tc_splits).
+// out in (tc_splits). wait_limit: polls of a product's completion (kTcWaitLimit;
+// a test lets it run out), after which kStatusTensorWait is set.
 static __global__ void __launch_bounds__(kTcBlock, kTcCtas)
 k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint32_t* __restrict__ cand_ids,
            const uint32_t* __restrict__ seg_off, const uint32_t* __restrict__ seg_cnt,
            const unsigned long long* __restrict__ total_ptr, unsigned long long arena_cap, int* __restrict__ status,
            AlignRes* __restrict__ out, unsigned long long* __restrict__ work_count,
-           const uint32_t* __restrict__ mirror, unsigned int* __restrict__ cursor, uint32_t splits, TcLayout lay) {
+           const uint32_t* __restrict__ mirror, unsigned int* __restrict__ cursor, uint32_t splits, TcLayout lay,
+           uint32_t wait_limit) {
     extern __shared__ __align__(128) unsigned char tsm[];
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ uint32_t s_tmem, s_next;
@@ -374,9 +378,11 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                         if (mirn != kMirrorSkip) Lcn = r.len[cn];
                         have_len = true;
                     }
-                    if (warp == 0) bad |= !tc05::mbar_wait(&s_bar, phase);    // one warp polls
+                    if (warp == 0) bad = !tc05::mbar_wait(&s_bar, phase, wait_limit);    // one warp polls
                     phase ^= 1u;
-                    __syncthreads();
+                    // after a wait that ran out no product follows: the
+                    // barrier's parity tells one unfinished product only
+                    if (__syncthreads_or(bad)) goto done;
                     tc05::fence_after_sync();
 #pragma unroll 1
                     for (int t = 0; t < nt; ++t) {
@@ -439,7 +445,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                     }
                 }
                 tc05::fence_before_sync();
-                if (__syncthreads_or(bad)) goto done;
+                __syncthreads();
                 // ---- exact counts of the possible shifts; of every shift when
                 //      there are more than the list holds ----
                 {
@@ -543,7 +549,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
 done:
     if (__syncthreads_or(bad)) {
         if (tid == 0) atomicOr(status, kStatusTensorWait);
-        tc05::mbar_wait(&s_bar, phase ^ 1u);            // products in flight end before their memory is released
+        tc05::mbar_wait(&s_bar, phase ^ 1u);            // the product in flight ends before its memory is released
     }
     if (work_count) {
 #pragma unroll

@@ -1047,7 +1047,7 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
                     o, r, first, count, ctx->d_cand_ids.as<uint32_t>(), ctx->d_seg_off.as<uint32_t>(),
                     ctx->d_seg_cnt.as<uint32_t>(), counters, cap, status, ctx->d_ares.as<AlignRes>(), counters + 3,
                     tu.pair_mirror ? ctx->d_pair_work.as<uint32_t>() : nullptr,
-                    reinterpret_cast<unsigned int*>(counters + 11), splits, tcl);
+                    reinterpret_cast<unsigned int*>(counters + 11), splits, tcl, kTcWaitLimit);
                 EQ(cudaGetLastError(), "k_align_tc");
                 ++launches;
             }

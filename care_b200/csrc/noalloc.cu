@@ -196,7 +196,7 @@ extern "C" int care_b200_correct_range_noalloc(const care_b200_options* opt, con
         const uint32_t splits = tc_splits(num_anchors, resident);
         k_align_tc<<<std::min<unsigned>(num_anchors * splits, resident), kTcBlock, tcl.total, st>>>(
             o, r, first_anchor, num_anchors, cand_ids, seg_off, seg_cnt, counters, kNoAllocMaxPairs, dstatus, ares,
-            nullptr, nullptr, reinterpret_cast<unsigned int*>(scratch + kOffCursor), splits, tcl);
+            nullptr, nullptr, reinterpret_cast<unsigned int*>(scratch + kOffCursor), splits, tcl, kTcWaitLimit);
     } else {
         // the pairs the candidate pass found size the alignment grid; a count
         // above the array's pair capacity ends the call here
