@@ -166,6 +166,8 @@ enum : int {
     kStatusCorrOverflow = 2,          // candidate-correction arena too small
     kStatusFeatOverflow = 8,          // decision-column arena too small
     kStatusTensorWait = 16,           // a tensor-core completion wait ran out
+    // results of an earlier stage are missing: later stages leave at once
+    kStatusIncomplete = kStatusCandOverflow | kStatusTensorWait,
 };
 
 // MurmurHash3 64-bit finalizer (the published fmix64), as used by the

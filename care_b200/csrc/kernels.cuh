@@ -1662,7 +1662,7 @@ k_msa(DevOptions o, DevReads r, uint32_t first, uint32_t count, MsaGrid grid, co
       const uint32_t* __restrict__ seg_cnt, const AlignRes* __restrict__ ares,
       CandRec* __restrict__ recs, MsaOut out, int* __restrict__ status) {
     if (blockIdx.x >= count) return;
-    if (*status & kStatusCandOverflow) return;   // batch is repeated with a larger arena
+    if (*status & kStatusIncomplete) return;     // unwritten candidates or alignments
     msa_anchor<BLOCK, QB, EMIT>(o, r, first, order ? order[blockIdx.x] : blockIdx.x, grid, cand_ids, seg_off,
                                 seg_cnt, ares, recs, out, status);
 }
@@ -1677,7 +1677,7 @@ k_msa_queue(DevOptions o, DevReads r, uint32_t first, uint32_t count, MsaGrid gr
             const AlignRes* __restrict__ ares, CandRec* __restrict__ recs, MsaOut out,
             int* __restrict__ status) {
     __shared__ uint32_t s_item;
-    if (*status & kStatusCandOverflow) return;
+    if (*status & kStatusIncomplete) return;
     for (;;) {
         __syncthreads();                      // the previous anchor is done with shared memory
         if (threadIdx.x == 0) s_item = atomicAdd(cursor, 1u);

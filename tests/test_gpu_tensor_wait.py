@@ -1,6 +1,7 @@
 """The completion wait of the tensor-core alignment running out: the kernel
 ends with its status set, writes no result of the product it gave up on, and
-leaves the GPU as a later launch needs it. The limit of the wait is set to
+leaves the GPU as a later launch needs it; the MSA behind it leaves at once
+(the alignments are unwritten). The limit of the wait is set to
 zero polls; the products themselves complete."""
 import ctypes
 import os
@@ -28,25 +29,28 @@ def build():
     return ctypes.CDLL(OUT)
 
 
-def _run(lib, rows, n, L, limit, grid):
+def _run(lib, rows, n, L, limit, grid, queue):
     res = np.zeros((n * (n - 1), 8), np.uint8)
+    corrected = np.zeros(n, np.uint8)
     status = ctypes.c_int(-1)
-    assert lib.gpu_align_with_limit(rows.ctypes.data_as(ctypes.c_void_p), n, L, ctypes.c_uint32(limit), grid,
-                                    res.ctypes.data_as(ctypes.c_void_p), ctypes.byref(status)) == 0
-    return status.value, res
+    assert lib.gpu_align_with_limit(rows.ctypes.data_as(ctypes.c_void_p), n, L, ctypes.c_uint32(limit), grid, queue,
+                                    res.ctypes.data_as(ctypes.c_void_p), corrected.ctypes.data_as(ctypes.c_void_p),
+                                    ctypes.byref(status)) == 0
+    return status.value, res, corrected
 
 
 # reads of 256 bases take several products per list of candidates, those of 60 one
 @pytest.mark.gpu
-@pytest.mark.parametrize("L,n", [(60, 9), (256, 40)])
-def test_wait_that_runs_out(L, n):
+@pytest.mark.parametrize("L,n,queue", [(60, 9, 0), (256, 40, 0), (256, 40, 1)])
+def test_wait_that_runs_out(L, n, queue):
     lib = build()
     rng = np.random.default_rng(L)
     rows = rng.integers(0, 1 << 32, (n, (L + 15) // 16), dtype=np.uint32)
     rows[1::2] = rows[0::2][: n // 2]                 # copies: pairs that align
-    status, res = _run(lib, rows, n, L, 0, 3)
+    status, res, corrected = _run(lib, rows, n, L, 0, 3, queue)
     assert status == TENSOR_WAIT
     assert (res == 0x5A).all()                        # no result
-    status, res = _run(lib, rows, n, L, LIMIT, 3)
-    assert status == 0
+    assert (corrected == 0x5A).all()                  # the MSA looked at no anchor
+    status, res, corrected = _run(lib, rows, n, L, LIMIT, 3, queue)
+    assert status == 0 and (corrected != 0x5A).all()
     assert res[0, 6] == 1 and not res[0, :2].any()    # read 1 is a copy of read 0: forward, shift 0
