@@ -819,18 +819,14 @@ struct MsaArgs {
     MsaGrid mgrid;                             // the staged rows' grid
 };
 
-// prepare (host only: attributes, occupancy) or launch one MSA variant
+// prepare (host only: occupancy) or launch one MSA variant
 template <int B, int QB, bool E>
 cudaError_t msa_go(MsaArgs& a, bool prepare, cudaStream_t st) {
     constexpr int kMany = B == 128 && !E ? kMsaManyCtas : (E ? 768 : 1024) / B;
     const bool many = msa_many_ctas(a.smem, a.count, a.sms);
     if (prepare) {
-        cudaError_t e = many ? cudaFuncSetAttribute(k_msa<B, QB, E, kMany>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem)
-                             : cudaFuncSetAttribute(k_msa<B, QB, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_msa_queue<B, QB, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem);
         int nb = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_msa_queue<B, QB, E>, B, a.smem);
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_msa_queue<B, QB, E>, B, a.smem);
         a.grid = (int)std::min<uint64_t>(a.count, (uint64_t)a.sms * (uint64_t)std::max(nb, 1));
         return e;
     }
@@ -872,7 +868,7 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
     while ((size_t)1 << set_log2 < (tmax * 4 + 2) / 3 + 1) set_log2++;
     const int groups = kCandBlock / h;
     const size_t cand_smem = CandSmem::total(ctx->max_len, groups, h, ctx->seq_pitch, 1 << set_log2);
-    if (cand_smem > 227 * 1024) return fail(ctx, CARE_B200_ELIMIT, "num_maps * threshold too large for the de-duplication set");
+    if (cand_smem > kCandSmemLimit) return fail(ctx, CARE_B200_ELIMIT, "num_maps * threshold too large for the de-duplication set");
     if (ctx->sms == 0) CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->opt.device), "attr");
     // the main candidate pass uses a set of at most 2^cand_set_log2 entries
     // (high occupancy); anchors with more unique ids than half of it are
@@ -881,11 +877,11 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
     const int set_log2_main = spill ? tu.cand_set_log2 : set_log2;
     const size_t cand_smem_main = CandSmem::total(ctx->max_len, groups, h, ctx->seq_pitch, 1 << set_log2_main);
     CK(cudaFuncSetAttribute(k_candidates<kCandBlock>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)cand_smem_main), "smem attr");
+                            (int)kCandSmemLimit), "smem attr");
     int spill_grid = 0;
     if (spill) {
         CK(cudaFuncSetAttribute(k_candidates_spill<kCandBlock>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)cand_smem), "smem attr");
+                                (int)kCandSmemLimit), "smem attr");
         int nb = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_candidates_spill<kCandBlock>, kCandBlock, cand_smem),
            "occupancy");
@@ -927,7 +923,6 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
     const bool tc = tc_applies(o.max_error_rate, o.min_overlap, o.min_overlap_ratio) && !ctx->count_words &&
                     tu.align_warp == 0 && !classes;
     const TcLayout tcl = tc_layout(ctx->max_len, ctx->opt.min_overlap, ctx->opt.min_overlap_ratio);
-    if (tc) CK(cudaFuncSetAttribute(k_align_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcl.total), "smem attr");
     const int qb = ctx->has_qual ? ctx->opt.quality_bits : 0;
     const MsaGrid mgrid = msa_grid(ctx->max_len, qb, o.correct_candidates, o.new_columns);
     const size_t msmem = msa_smem_bytes(mgrid, ctx->max_len, emit);

@@ -27,6 +27,12 @@ __constant__ float c_qweight[256];    // QualityScoreConversion table (qualitysc
 // ---------------------------------------------------------------------------
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 
+// Shared memory that a launch of k_candidates or k_candidates_spill may take.
+// The limit is set to this at every launch: it belongs to the function on the
+// device, and a limit of each call's own size could fall below another
+// thread's between that thread's setting and its launch.
+constexpr size_t kCandSmemLimit = 227 * 1024 - 256;
+
 struct CandSmem {
     // dynamic shared memory layout, all offsets in bytes
     static __host__ __device__ size_t canon(int) { return 0; }
@@ -813,7 +819,7 @@ struct MsaGrid {
     int edge, words, wpg, rw, rows;
     uint32_t magic;                   // x / words as the high word of x * magic (words > 1)
 };
-__host__ __device__ inline MsaGrid msa_grid(int max_len, int qb, int correct_candidates, int new_columns) {
+__host__ __device__ constexpr MsaGrid msa_grid(int max_len, int qb, int correct_candidates, int new_columns) {
     MsaGrid g{};
     const int nc = new_columns < 0 ? 0 : new_columns > kMaxLen ? kMaxLen : new_columns;
     g.edge = correct_candidates ? (nc + 15) / 16 : 0;
@@ -830,13 +836,27 @@ __host__ __device__ inline MsaGrid msa_grid(int max_len, int qb, int correct_can
 // candidates), per anchor position the support and the four counts, with
 // decision rows three column weights, then the coverage, the column list and
 // the bases of the grid's columns. Every part starts on a 16-byte boundary.
-__host__ __device__ inline size_t msa_round16(size_t x) { return (x + 15) & ~(size_t)15; }
-__host__ __device__ inline size_t msa_smem_bytes(const MsaGrid& g, int max_len, bool emit) {
+__host__ __device__ constexpr size_t msa_round16(size_t x) { return (x + 15) & ~(size_t)15; }
+__host__ __device__ constexpr size_t msa_smem_bytes(const MsaGrid& g, int max_len, bool emit) {
     const size_t cols = 16 * (size_t)g.words;
     return msa_round16((size_t)(g.rows + 1) * g.rw * 4) + msa_round16((size_t)max_len * 4) + (size_t)max_len * 8 +
            8 * (size_t)(max_len & 1) + (emit ? msa_round16((size_t)3 * max_len * 4) : 0) +
            msa_round16((size_t)max_len * 2) + msa_round16(cols * 2) + cols;
 }
+// the most that any read length, quality encoding and edge takes
+constexpr size_t msa_smem_most() {
+    size_t most = 0;
+    for (int qb = 0; qb <= 8; qb = qb == 0 ? 1 : 2 * qb)
+        for (int len = 1; len <= kMaxLen; ++len)
+            for (int nc = 0; nc <= kMaxLen; nc += 16) {
+                const size_t n = msa_smem_bytes(msa_grid(len, qb, 1, nc), len, true);
+                most = n > most ? n : most;
+            }
+    return most;
+}
+// With the static part (below 10 KB) no launch needs a raised limit, which
+// would be shared by all threads of the process.
+static_assert(msa_smem_most() + 10240 <= 48 * 1024, "the MSA fits the default limit");
 
 // reverse the 16 2-bit codes of a word, keeping each code's bits
 __device__ __forceinline__ uint32_t rev2(uint32_t w) {

@@ -177,8 +177,8 @@ extern "C" int care_b200_correct_range_noalloc(const care_b200_options* opt, con
     int set_log2 = 6;                 // at least 64 entries: the set and the sort pad to 64 and 32
     while ((size_t)1 << set_log2 < (tmax * 4 + 2) / 3 + 1) set_log2++;
     const size_t cand_smem = CandSmem::total(r.max_len, 128 / h, h, r.seq_pitch, 1 << set_log2);
-    if (cand_smem > 227 * 1024) return CARE_B200_ELIMIT;
-    if (cudaFuncSetAttribute(k_candidates<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cand_smem) != cudaSuccess)
+    if (cand_smem > kCandSmemLimit) return CARE_B200_ELIMIT;
+    if (cudaFuncSetAttribute(k_candidates<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCandSmemLimit) != cudaSuccess)
         return CARE_B200_ECUDA;
     k_candidates<128><<<num_anchors, 128, cand_smem, st>>>(
         o, r, static_cast<const TableDesc*>(tables->descs), static_cast<const Slot*>(tables->slots), tables->values,
@@ -190,8 +190,6 @@ extern "C" int care_b200_correct_range_noalloc(const care_b200_options* opt, con
         const TcLayout tcl = tc_layout(r.max_len, o.min_overlap, o.min_overlap_ratio);
         int sms = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return CARE_B200_ECUDA;
-        if (cudaFuncSetAttribute(k_align_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcl.total) != cudaSuccess)
-            return CARE_B200_ECUDA;
         const unsigned resident = (unsigned)(sms * tc_ctas(tcl));
         const uint32_t splits = tc_splits(num_anchors, resident);
         k_align_tc<<<std::min<unsigned>(num_anchors * splits, resident), kTcBlock, tcl.total, st>>>(
@@ -225,15 +223,9 @@ extern "C" int care_b200_correct_range_noalloc(const care_b200_options* opt, con
     const int qb = !o.use_quality ? 0 : o.quality_bits == 1 ? 1 : o.quality_bits == 2 ? 2 : 8;
     const MsaGrid mgrid = msa_grid(r.max_len, qb, 0, 0);
     const size_t msmem = msa_smem_bytes(mgrid, r.max_len, false);
-#define LAUNCH_MSA(QB)                                                                                   \
-    do {                                                                                                  \
-        if (cudaFuncSetAttribute(k_msa<128, QB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem) \
-            != cudaSuccess)                                                                               \
-            return CARE_B200_ECUDA;                                                                       \
-        k_msa<128, QB><<<num_anchors, 128, msmem, st>>>(o, r, first_anchor, num_anchors, mgrid, nullptr,     \
-                                                        cand_ids, seg_off, seg_cnt, ares, recs, mo,       \
-                                                        dstatus);                                         \
-    } while (0)
+#define LAUNCH_MSA(QB)                                                                                     \
+    k_msa<128, QB><<<num_anchors, 128, msmem, st>>>(o, r, first_anchor, num_anchors, mgrid, nullptr, cand_ids, \
+                                                    seg_off, seg_cnt, ares, recs, mo, dstatus)
     if (!o.use_quality) LAUNCH_MSA(0);
     else if (o.quality_bits == 1) LAUNCH_MSA(1);
     else if (o.quality_bits == 2) LAUNCH_MSA(2);

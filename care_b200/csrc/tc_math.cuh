@@ -31,7 +31,7 @@ struct TcLayout {
     uint32_t aw, ar, q, top, b, fw, total;
 };
 
-inline TcLayout tc_layout(int max_len, int min_overlap, float min_overlap_ratio) {
+constexpr TcLayout tc_layout(int max_len, int min_overlap, float min_overlap_ratio) {
     TcLayout t{};
     t.W = 2 * ((max_len + 31) / 32);
     t.RS = (t.W + 1) | 1;
@@ -59,6 +59,12 @@ inline TcLayout tc_layout(int max_len, int min_overlap, float min_overlap_ratio)
     t.total = at;
     return t;
 }
+
+// The widest layout, with the static part, needs no raised shared-memory limit.
+// Such a limit belongs to the function on the device, not to a context: one set
+// per call to the call's own size could fall below another thread's between
+// that thread's setting and its launch.
+static_assert(tc_layout(kMaxLen, 1, 0.0f).total + 8192 <= 48 * 1024, "the alignment fits the default limit");
 
 // CTAs of the alignment that share an SM: its tensor memory, its shared memory
 // (8 KB of a CTA's part is static or reserved).
