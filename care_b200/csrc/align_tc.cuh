@@ -43,6 +43,7 @@
 namespace careb200 {
 
 constexpr uint32_t kTcWaitLimit = 1u << 22;
+constexpr int kTcGaveUp = 1 << 30;      // in place of the number of listed shifts: the wait ran out
 
 // Whether the tensor-core alignment takes these options.
 inline bool tc_applies(float max_error_rate, int min_overlap, float min_overlap_ratio) {
@@ -104,6 +105,16 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
+// 8 consecutive fp32 columns of this thread's tensor-memory lane
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
 // true in one lane of a converged warp
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
@@ -118,8 +129,8 @@ __device__ __forceinline__ uint32_t tc_desc_hi(uint32_t sbo) { return (sbo >> 4)
 // its shifts, then per product of up to 32 candidates (i) their packed rows,
 // both orientations, as operand columns, (ii) one tcgen05 product per
 // 128-shift tile, (iii) every sum against its shift's threshold (a warp reads
-// its 32 shifts of all columns), the possible ones listed, (iv) their exact
-// counts and a minimum per column, (v) the orientation, the pair flag and the
+// its 32 shifts of all columns), the possible ones listed (in a bit each when
+// there are too many), (iv) their exact counts and a minimum per column, (v) the orientation, the pair flag and the
 // AlignRes. The next anchor's segment, ids and lengths load meanwhile.
 // mirror (may be null): k_mirror_index's array; a leading pair also writes
 // its mirror's result. splits: parts that an anchor's candidates are handed
@@ -351,13 +362,10 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                 __syncthreads();
                 // ---- products, thresholds ----
                 const int nbuf = 2 * nI <= kTcCols / 2 ? 2 : 1;
+                int kept = 0;
 #pragma unroll 1
                 for (int t0 = 0; t0 < ntiles; t0 += nbuf) {
                     const int nt = min(nbuf, ntiles - t0);
-                    if (t0) {                                 // the buffers' sums have been read
-                        tc05::fence_before_sync();
-                        __syncthreads();
-                    }
                     if (warp == 0 && elect_one()) {
                         tc05::fence_after_sync();
                         const uint32_t idesc = (1u << 4) | ((uint32_t)(2 * nI >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -378,11 +386,12 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                         if (mirn != kMirrorSkip) Lcn = r.len[cn];
                         have_len = true;
                     }
-                    if (warp == 0) bad = !tc05::mbar_wait(&s_bar, phase, wait_limit);    // one warp polls
+                    // one warp polls; after a wait that ran out no product
+                    // follows: the barrier's parity tells one unfinished
+                    // product only
+                    if (warp == 0 && !tc05::mbar_wait(&s_bar, phase, wait_limit)) s_nh = kTcGaveUp;
                     phase ^= 1u;
-                    // after a wait that ran out no product follows: the
-                    // barrier's parity tells one unfinished product only
-                    if (__syncthreads_or(bad)) goto done;
+                    __syncthreads();
                     tc05::fence_after_sync();
 #pragma unroll 1
                     for (int t = 0; t < nt; ++t) {
@@ -429,12 +438,14 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                                         uint32_t hits = 0u;
 #pragma unroll
                                         for (int e = 0; e < 8; ++e) if (v[8 * g + e] >= limit) hits |= 1u << e;
+                                        if (*(volatile int*)&s_nh > kTcHits) continue;    // the list has overflowed
+                                        int p = atomicAdd(&s_nh, __popc(hits));
                                         do {
                                             const int e = __ffs(hits) - 1;
                                             hits &= hits - 1u;
-                                            const int p = atomicAdd(&s_nh, 1);
                                             if (p < kTcHits)
                                                 s_hit[p] = (uint32_t)(q + 8 * g + e) | (uint32_t)(s + 512) << 16;
+                                            ++p;
                                         } while (hits);
                                     }
                                 }
@@ -443,30 +454,21 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                         if (uniform) scan_tile(std::true_type{});
                         else scan_tile(std::false_type{});
                     }
-                }
-                tc05::fence_before_sync();
-                __syncthreads();
-                // ---- exact counts of the possible shifts; of every shift when
-                //      there are more than the list holds ----
-                {
+                    tc05::fence_before_sync();
+                    __syncthreads();
+                    // ---- exact counts of the listed shifts, once the last
+                    //      sums are read (of an overflowing round, of those
+                    //      kept from the rounds before): four lanes per shift,
+                    //      each every fourth word ----
                     const int nh = s_nh;
-                    const bool all = nh > kTcHits;
-                    const int span = ntiles * 128;
-                    const int work = all ? 2 * n * span : nh;
-                    // four lanes per shift, each every fourth word
+                    if (nh <= kTcHits && t0 + nbuf < ntiles) { kept = nh; continue; }
+                    if (nh >= kTcGaveUp) { bad = true; goto done; }
+                    const int work = nh > kTcHits ? kept : nh;
+                    kept = 0;
 #pragma unroll 1
                     for (int k0 = 8 * warp; k0 < work; k0 += kTcBlock / 4) {
-                        const int k = min(k0 + (lane >> 2), work - 1);
-                        int col, sh;
-                        if (all) {
-                            col = k / span;
-                            sh = smax - (k - col * span);
-                            if (col >= n) col += nI - n;
-                        } else {
-                            const uint32_t hv = s_hit[k];
-                            col = (int)(hv & 0xFFFFu);
-                            sh = (int)(hv >> 16) - 512;
-                        }
+                        const uint32_t hv = s_hit[min(k0 + (lane >> 2), work - 1)];
+                        const int col = (int)(hv & 0xFFFFu), sh = (int)(hv >> 16) - 512;
                         const int rev = col >= nI;
                         const int it = col - rev * nI;
                         const int L = s_len[i0 + it];
@@ -485,6 +487,71 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
                             const uint32_t sc = (uint32_t)(mm + La + L - 2 * ov) << 10;
                             atomicMin(&s_key[rev][it], sc | tc_rank(sh));
                             if (mirror && ov >= minov_of(L)) atomicMin(&s_key[2 + rev][it], sc | tc_rank(tc_mirror_shift(sh, rev, La, L)));
+                        }
+                    }
+                    if (nh <= kTcHits) continue;
+                    // ---- more possible shifts than the list holds (reads of
+                    //      short tandem repeats): the round's possible shifts
+                    //      as a bit each, from the sums, then each column's
+                    //      groups of 32 shifts by falling overlap, a lane per
+                    //      shift, up to the mismatches that still improve on
+                    //      the column's best. Against counts of all shifts of
+                    //      the product, alignment ms with 2, 20 and 60 % of the
+                    //      genome in repeats of 1-6 bases: 300k reads of 100
+                    //      bases 7.9 -> 4.9 and 31.5 -> 7.6, 200k of 150 bases
+                    //      146 -> 24 (thread scan 5.7, 6.3, 12.9) ----
+                    __syncthreads();                          // the list's words become the bits
+                    if (tid == 0) s_nh = 0;
+#pragma unroll 1
+                    for (int t = 0; t < nt; ++t) {
+                        const int s = smax - 127 - 128 * (t0 + t) + srow;
+                        const int u = max(s, 0);
+                        const float c1 = kappa * (float)(La - u) + kTcSlack, c2 = kappa * (float)(s - u) + kTcSlack;
+                        const float cmin = s >= smin ? kappa * (float)minov + kTcSlack : 1e9f;
+                        const uint32_t col0 = tmem + ((uint32_t)warp << 21) + (uint32_t)(t * (kTcCols / 2));
+#pragma unroll 1
+                        for (int q = 0; q < 2 * nI; q += 8) {
+                            float v[8];
+                            tmem_ld8(col0 + q, v);
+                            const float* kl = &s_kl[q - (q >= nI ? nI : 0)];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                const uint32_t b = __ballot_sync(0xffffffffu, v[e] >= fmaxf(fminf(c1, kl[e] + c2), cmin));
+                                if (lane == 0) s_hit[4 * (t * 2 * nI + q + e) + warp] = b;
+                            }
+                        }
+                    }
+                    tc05::fence_before_sync();
+                    __syncthreads();
+#pragma unroll 1
+                    for (int en = warp; en < nt * 2 * nI; en += kTcWarps) {
+                        const uint32_t bits = s_hit[4 * en + tc_shift_word(lane)] >> tc_shift_bit(lane, 0) & 0x55u;
+                        if (!__any_sync(0xffffffffu, bits != 0u)) continue;
+                        const int t = en >= 2 * nI, col = en - t * 2 * nI, rev = col >= nI, it = col - rev * nI;
+                        const int L = s_len[i0 + it], minl2 = mirror ? minov_of(L) : 0;
+                        const int s0 = smax - 127 - 128 * (t0 + t);
+                        const uint32_t ca = lay.fw + 4u * (uint32_t)(it * RS), an = rev ? lay.ar : lay.aw;
+#pragma unroll 1
+                        for (int k = 0; k < 7; ++k) {
+                            const int g = tc_group(s0, k);
+                            if ((unsigned)g > 3u || !__any_sync(0xffffffffu, (bits >> 2 * g) & 1u)) continue;
+                            const int sh = s0 + 32 * g + lane, ov = tc_overlap(sh, La, L);
+                            const bool mirrored = mirror && ov >= minl2;
+                            const int cap = ov < minov ? 0 : tc_cap(ov, mex_of(ov), La, L, *(volatile uint32_t*)&s_key[rev][it],
+                                                                    mirrored, *(volatile uint32_t*)&s_key[2 + rev][it]);
+                            if (((bits >> 2 * g) & 1u) && cap > 0) {
+                                const int sv = rev ? La - L - sh : sh;
+                                const bool pos = sv >= 0;
+                                const int mm = tc_mismatches_below(reinterpret_cast<const uint32_t*>(tsm + (pos ? an : ca)),
+                                                                   reinterpret_cast<const uint32_t*>(tsm + (pos ? ca : an)),
+                                                                   pos ? sv : -sv, ov, cap);
+                                if (mm < cap) {
+                                    const uint32_t sc = (uint32_t)(mm + La + L - 2 * ov) << 10;
+                                    atomicMin(&s_key[rev][it], sc | tc_rank(sh));
+                                    if (mirrored) atomicMin(&s_key[2 + rev][it], sc | tc_rank(tc_mirror_shift(sh, rev, La, L)));
+                                }
+                            }
+                            __syncwarp();
                         }
                     }
                 }
@@ -547,7 +614,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
         Lc = Lcn;
     }
 done:
-    if (__syncthreads_or(bad)) {
+    if (bad) {
         if (tid == 0) atomicOr(status, kStatusTensorWait);
         tc05::mbar_wait(&s_bar, phase ^ 1u);            // the product in flight ends before its memory is released
     }

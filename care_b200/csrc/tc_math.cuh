@@ -13,7 +13,10 @@ constexpr int kTcWindow = kTcBlock;     // candidates looked at at a time
 constexpr int kTcCols = 64;             // tensor-memory columns of a CTA
 constexpr int kTcCtas = 512 / kTcCols;  // CTAs that the tensor memory of an SM holds
 constexpr int kTcMate = 192;            // ids of the mate's list held in shared memory
-constexpr int kTcHits = 256;            // possible (shift, column) waiting for their exact count
+// Possible (shift, column) waiting for their exact count; with more of them the
+// same words hold a bit for each shift of a round's sums.
+constexpr int kTcHits = 256;
+static_assert(kTcHits == 4 * kTcCols, "four words of shifts per column of sums");
 // A random pair of bases differs in its high bit with probability 1/2, so up
 // to this rate a possible shift is rare; above it the thread scan runs.
 constexpr float kTcMaxErrorRate = 0.30f;
@@ -174,6 +177,48 @@ CB_HD int tc_mismatches(const uint32_t* x, const uint32_t* y, int t, int ov, int
     return mm;
 }
 
+// The same, but any value from cap on when they are not below cap.
+CB_HD int tc_mismatches_below(const uint32_t* x, const uint32_t* y, int t, int ov, int cap) {
+    const int w0 = t >> 4, r = 2 * (t & 15);
+    int mm = 0;
+    const uint32_t* xp = x + w0;
+    uint32_t hi = xp[0];
+    int left = ov;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+    for (; left >= 32 && mm < cap; left -= 32) {       // two words a step
+        const uint32_t m = xp[1], lo = xp[2];
+        uint32_t d0 = funnel_l(m, hi, r) ^ y[0], d1 = funnel_l(lo, m, r) ^ y[1];
+        hi = lo;
+        xp += 2;
+        y += 2;
+        d0 = (d0 | (d0 >> 1)) & 0x55555555u;
+        d1 = (d1 | (d1 >> 1)) & 0x55555555u;
+        mm += popc32(d0 | d1 << 1);
+    }
+    if (left >= 32) return mm;
+    for (; left > 0 && mm < cap; left -= 16) {
+        const uint32_t lo = xp[1];
+        uint32_t d = funnel_l(lo, hi, r) ^ y[0];
+        hi = lo;
+        ++xp;
+        ++y;
+        d = (d | (d >> 1)) & 0x55555555u;
+        if (left < 16) d &= ~(0xFFFFFFFFu >> (2 * left));
+        mm += popc32(d);
+    }
+    return mm;
+}
+
+// Mismatches from which on a shift of overlap ov can no longer improve a column
+// whose best keys are `key` (for the mirror, where the overlap is long enough
+// for it, `mkey`): a shift of as many mismatches and a lower rank still can.
+CB_HD int tc_cap(int ov, int mex, int La, int Lc, uint32_t key, bool mirrored, uint32_t mkey) {
+    const uint32_t best = max(key >> 10, mirrored ? mkey >> 10 : 0u);
+    return min(mex, (int)best - (La + Lc - 2 * ov) + 1);
+}
+
 // Rank of shift s in the scan order 0, 1, ..., then -1, -2, ... (A's shift s
 // is -s for (C, A)). Keys are score << 10 | rank; ranks and scores stay below
 // 1024.
@@ -200,6 +245,17 @@ CB_HD ShdResult tc_result(uint32_t key, int La, int Lc) {
 // The row of a 128-shift tile as a shift relative to the tile's first: the
 // 8-row group m / 8 holds shifts m / 8 + 16 * (m % 8).
 CB_HD int tc_row_shift(int m) { return (m >> 3) + 16 * (m & 7); }
+
+// Its bit in a column's four words (one per warp) as the shift's place in the
+// tile: lane l of group g (the shifts 32 g + l) finds it in word (l % 16) / 4.
+CB_HD int tc_shift_word(int l) { return (l & 15) >> 2; }
+CB_HD int tc_shift_bit(int l, int g) { return 8 * (l & 3) + (l >> 4) + 2 * g; }
+// The k-th of a tile's four groups from the one nearest shift 0 outwards (the
+// overlaps fall that way); outside 0 .. 3 there is none. s0: the first shift.
+CB_HD int tc_group(int s0, int k) {
+    const int at = -s0 >> 5;
+    return (at < 0 ? 0 : at > 3 ? 3 : at) + ((k & 1) ? (k + 1) >> 1 : -(k >> 1));
+}
 
 // Chunk x of the anchor's operand bytes: 16 bytes from base q0 + 16 * x on,
 // q0 = smax - 127 - 128 * (tiles - 1), zeros outside the read.

@@ -14,8 +14,10 @@ static float e4m3(uint8_t b) { return b == 0x38 ? 1.0f : b == 0xB8 ? -1.0f : b =
 // rows: n candidates of `pitch` words. out: 22 ints per candidate -- score,
 // overlap, shift, nops, valid of (A, C), of (A, rc C), of (C, A) and of (C, rc
 // A) (for a candidate not shorter than the anchor), then the orientations of
-// (A, C) and (C, A). per_column: the threshold form of mixed lengths. Returns the
-// possible shifts listed, -1 on a byte no operand holds, -2 on an index past
+// (A, C) and (C, A). per_column: 1 the threshold form of mixed lengths, 2 that
+// form and the counts of a list that overflows (a bit per possible shift,
+// counted in groups of 32 by falling overlap, up to what still improves on the
+// best). Returns the possible shifts listed, -1 on a byte no operand holds, -2 on an index past
 // a buffer.
 extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch, const int* len, int n, int max_len,
                      int min_overlap, float rate, float ratio, float est, int per_column, int* out) {
@@ -68,7 +70,8 @@ extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch,
     const float kappa = 1.0f - 2.0f * rate;
     int hits = 0;
     const int K = 32 * ((maxl + 31) / 32);
-    for (int t = 0; t < ntiles; ++t)
+    for (int t = 0; t < ntiles; ++t) {
+        std::vector<uint32_t> bits((size_t)4 * 2 * n, 0u);       // a column's words, one per warp
         for (int m = 0; m < 128; ++m) {
             const int s = smax - 127 - 128 * t + tc_row_shift(m);
             for (int col = 0; col < 2 * n; ++col) {
@@ -96,6 +99,10 @@ extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch,
                 }
                 if (!(d >= thr)) continue;
                 ++hits;
+                if (per_column == 2) {
+                    bits[(size_t)4 * col + (m >> 5)] |= 1u << (m & 31);
+                    continue;
+                }
                 const int ov = tc_overlap(s, La, Lc);
                 if (ov < minov) continue;
                 // the reverse complement's shift, seen from the anchor's reverse complement
@@ -116,6 +123,39 @@ extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch,
                 kc = kc < m ? kc : m;
             }
         }
+        const int s0 = smax - 127 - 128 * t;
+        for (int col = 0; per_column == 2 && col < 2 * n; ++col) {
+            const int rev = col >= n, it = col - rev * n, Lc = len[it];
+            const uint32_t *cr = &fw[it * RS], *an = rev ? ar.data() : aw.data();
+            const int lc = f2i_rz(fmul_rn((float)Lc, ratio)), minlc = min_overlap > lc ? min_overlap : lc;
+            int seen = 0;
+            for (int k = 0; k < 7; ++k) {
+                const int g = tc_group(s0, k);
+                if ((unsigned)g > 3u) continue;
+                seen |= 1 << g;
+                uint32_t ka = key[rev * n + it], kc = key[(2 + rev) * n + it];
+                const uint32_t ka0 = ka, kc0 = kc;               // what the group's lanes see
+                for (int lane = 0; lane < 32; ++lane) {
+                    const int s = s0 + 32 * g + lane, ov = tc_overlap(s, La, Lc);
+                    if (tc_row_shift(32 * tc_shift_word(lane) + tc_shift_bit(lane, g)) != 32 * g + lane) return -2;
+                    if (!((bits[(size_t)4 * col + tc_shift_word(lane)] >> tc_shift_bit(lane, g)) & 1u)) continue;
+                    const bool mirrored = ov >= minlc;
+                    const int cap = ov < minov ? 0 : tc_cap(ov, f2i_rz(fmul_rn((float)ov, rate)), La, Lc, ka0, mirrored, kc0);
+                    if (cap <= 0) continue;
+                    const int sv = rev ? La - Lc - s : s;
+                    const int mm = sv >= 0 ? tc_mismatches_below(an, cr, sv, ov, cap) : tc_mismatches_below(cr, an, -sv, ov, cap);
+                    if (mm >= cap) continue;
+                    const uint32_t sc = (uint32_t)(mm + La + Lc - 2 * ov) << 10;
+                    const uint32_t x = sc | tc_rank(s), y = sc | tc_rank(tc_mirror_shift(s, rev, La, Lc));
+                    ka = ka < x ? ka : x;
+                    if (mirrored) kc = kc < y ? kc : y;
+                }
+                key[rev * n + it] = ka;
+                key[(2 + rev) * n + it] = kc;
+            }
+            if (seen != 15) return -2;
+        }
+    }
     for (int it = 0; it < n; ++it) {
         const int L = len[it];
         const ShdResult rs[4] = {tc_result(key[it], La, L), tc_result(key[n + it], La, L),

@@ -123,6 +123,41 @@ def test_operands_and_results_match_the_oracle(lib, seed):
                     assert list(o[5 * k:5 * k + 5]) == [x.score, x.overlap, x.shift, x.nops, x.valid]
 
 
+@pytest.mark.parametrize("seed", range(60))
+def test_counts_of_an_overflowing_list(lib, seed):
+    """The form that counts a column's possible shifts from their bits and
+    stops at what no longer improves, against the count of every possible
+    shift: tandem repeats with ties, errors and unique ends."""
+    rng = random.Random(900 + seed)
+    La = FIXED[seed % len(FIXED)]
+    n = rng.choice([1, 5, 8])
+    lens = [La if seed % 2 else rng.randint(16, 256) for _ in range(n)]
+    mo, ratio, rate = rng.choice([30, 1, 12]), rng.choice([0.3, 0.0]), rng.choice([0.2, 0.3, 0.05])
+    unit = _rand(rng, 1 + seed % 7)
+    reads = []
+    for L in [La] + lens:
+        at = rng.randrange(len(unit))
+        r = (unit * 300)[at:at + L]
+        if rng.random() < 0.5:                           # an end outside the repeat
+            k = rng.randint(0, L)
+            r = r[:k] + _rand(rng, L - k)
+        r = _mutate(rng, r, rng.choice([0, 0, 2, L // 12]))
+        reads.append(_rc(r) if rng.random() < 0.3 else r)
+    max_len = max([La] + lens)
+    pitch = (max_len + 15) // 16
+    rows = np.stack([_enc(c, pitch) for c in reads[1:]])
+    ln = np.array(lens, np.int32)
+    out = []
+    for form in (1, 2):
+        o = np.zeros((n, 22), np.int32)
+        hits = lib.hd_tc(_enc(reads[0], 17).ctypes.data_as(ctypes.c_void_p), La, rows.ctypes.data_as(ctypes.c_void_p),
+                         pitch, ln.ctypes.data_as(ctypes.c_void_p), n, max_len, mo, ctypes.c_float(rate),
+                         ctypes.c_float(ratio), ctypes.c_float(0.06), form, o.ctypes.data_as(ctypes.c_void_p))
+        assert hits >= 0
+        out.append(o)
+    assert np.array_equal(out[0], out[1])
+
+
 def test_random_pairs_rarely_stay_possible(lib):
     """The one-bit sums rule out nearly every shift of unrelated reads: that
     is what makes the exact counts few."""

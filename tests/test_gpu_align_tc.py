@@ -85,6 +85,19 @@ def test_short_tandem_repeats(unit):
     _same(seqs, lengths, [(0, 160), (5, 20)], kmerlength=16, num_maps=8, estimated_coverage=400.0)
 
 
+@pytest.mark.parametrize("mirror", [0, 1])
+@pytest.mark.parametrize("lo,hi,unit", [(100, 100, 1), (150, 150, 2), (50, 250, 5), (256, 256, 4), (33, 64, 2)])
+def test_overflowing_lists(lo, hi, unit, mirror):
+    """Products with more possible shifts than the list holds, in one round of
+    sums and in several, beside unique sequence."""
+    rng = np.random.default_rng(unit + lo)
+    genome = np.concatenate([rng.integers(0, 4, 2 * hi), np.tile(rng.permutation(8)[:unit] & 3, 2 * hi // unit),
+                             rng.integers(0, 4, 2 * hi)])
+    seqs, lengths = _reads(3, 300, lo, hi, genome, rate=0.02)
+    _same(seqs, lengths, [(0, 300), (5, 20)], kmerlength=16, num_maps=8, estimated_coverage=400.0,
+          correct_candidates=1, tuning={"pair_mirror": mirror})
+
+
 @pytest.mark.parametrize("rate,overlap,ratio", [(0.0, 30, 0.3), (0.3, 1, 0.0), (0.30001, 30, 0.3), (0.2, 200, 1.0)])
 def test_option_edges(rate, overlap, ratio):
     genome = np.random.default_rng(9).integers(0, 4, 3000)
