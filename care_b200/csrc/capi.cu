@@ -918,10 +918,12 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
     // length classes of the alignment (not with mirror pairs, whose work list pairs equal lengths)
     const bool classes = tu.align_classes != 0 && tu.pair_mirror == 0;
     if (classes) CK(ctx->d_cls.ensure(64), "alloc");
-    // the tensor-core alignment, except for the statistics form and the
-    // mappings that ask for another scan
+    // the tensor-core alignment, except for the statistics form, the mappings
+    // that ask for another scan and the calls that the thread scan does faster
     const bool tc = tc_applies(o.max_error_rate, o.min_overlap, o.min_overlap_ratio) && !ctx->count_words &&
-                    tu.align_warp == 0 && !classes;
+                    tu.align_warp == 0 && !classes &&
+                    tc_faster(ctx->max_len, o.min_overlap, o.min_overlap_ratio, o.estimated_coverage, count,
+                              tu.pair_mirror != 0, 0.0f);
     const TcLayout tcl = tc_layout(ctx->max_len, ctx->opt.min_overlap, ctx->opt.min_overlap_ratio);
     const int qb = ctx->has_qual ? ctx->opt.quality_bits : 0;
     const MsaGrid mgrid = msa_grid(ctx->max_len, qb, o.correct_candidates, o.new_columns);

@@ -184,7 +184,9 @@ extern "C" int care_b200_correct_range_noalloc(const care_b200_options* opt, con
         o, r, static_cast<const TableDesc*>(tables->descs), static_cast<const Slot*>(tables->slots), tables->values,
         nullptr, first_anchor, num_anchors, set_log2, nullptr, nullptr, cand_ids, cand_anchor, seg_off, seg_cnt, counters, kNoAllocMaxPairs,
         dstatus);
-    if (tc_applies(o.max_error_rate, o.min_overlap, o.min_overlap_ratio)) {
+    // (the scan's route waits for the pair count: about 20 us)
+    if (tc_applies(o.max_error_rate, o.min_overlap, o.min_overlap_ratio) &&
+        tc_faster(r.max_len, o.min_overlap, o.min_overlap_ratio, o.estimated_coverage, num_anchors, false, 20.0f)) {
         // the grid follows the anchors; a pair count above the array's
         // capacity is in the status word, which every later kernel looks at
         const TcLayout tcl = tc_layout(r.max_len, o.min_overlap, o.min_overlap_ratio);

@@ -34,17 +34,23 @@ struct TcLayout {
     uint32_t aw, ar, q, top, b, fw, total;
 };
 
+// Shifts of the widest scan of one orientation.
+constexpr int tc_span(int max_len, int min_overlap, float min_overlap_ratio) {
+    int span = 1;
+    for (int la = 1; la <= max_len; ++la) {
+        const int lo = (int)((float)la * min_overlap_ratio);
+        const int m = lo > min_overlap ? lo : min_overlap, mo = m < max_len ? m : max_len;
+        const int n = la + max_len - 2 * mo + 1;
+        span = n > span ? n : span;
+    }
+    return span;
+}
+
 constexpr TcLayout tc_layout(int max_len, int min_overlap, float min_overlap_ratio) {
     TcLayout t{};
     t.W = 2 * ((max_len + 31) / 32);
     t.RS = (t.W + 1) | 1;
-    int span = 1;                       // shifts of the widest scan
-    for (int la = 1; la <= max_len; ++la) {
-        const int lo = (int)((float)la * min_overlap_ratio);
-        const int mo = lo > min_overlap ? lo : min_overlap;
-        const int n = la + max_len - 2 * mo + 1;
-        span = n > span ? n : span;
-    }
+    const int span = tc_span(max_len, min_overlap, min_overlap_ratio);
     t.tiles = (span + 127) / 128;
     t.XL = 7 + t.W + 8 * (t.tiles - 1);
     t.magic_w = (65536u + (uint32_t)t.W - 1) / (uint32_t)t.W;
@@ -81,6 +87,34 @@ inline int tc_ctas(const TcLayout& t) {
 inline uint32_t tc_splits(uint32_t anchors, uint32_t resident) {
     const uint32_t n = anchors ? resident / anchors : 1u;
     return n < 1u ? 1u : n > 8u ? 8u : n;
+}
+
+// Whether the tensor-core alignment is the faster one, from what the host
+// knows: an anchor costs it a chain of loads and barriers whatever its
+// candidates, and a product costs the same for few shifts as for many, so the
+// thread scan (k_align) is ahead where pairs are few or shifts are: short
+// reads, low coverage, a minimum overlap near the read's length. Costs fitted
+// to 200k reads of 36 to 250 bases at 5x to 40x (1.25 pairs per anchor and unit
+// of coverage) and to 128 to 4,000 anchors. Alignment ms, thread scan and
+// tensor cores: 36 bases 5x 0.16, 0.91; 50 bases 20x 0.89, 1.33; 60 bases 40x
+// 2.20, 2.17; 100 bases 5x 0.70, 1.18, 10x 1.31, 1.40, 20x 2.54, 1.95; 150
+// bases 5x 1.02, 1.26, 10x 1.95, 1.55; 150 bases 30x with a minimum overlap of
+// 135 1.18, 2.09, of 90 3.29, 2.40; 250 bases 5x 2.47, 1.91; 1,000 anchors of
+// 50 bases 5x 0.018, 0.022, of 70 bases 0.029, 0.022. fixed_us: what the scan's
+// route adds to a call.
+inline bool tc_faster(int max_len, int min_overlap, float min_overlap_ratio, float coverage, uint32_t anchors,
+                      bool mirror, float fixed_us) {
+    const int lo = (int)((float)max_len * min_overlap_ratio), mo = lo > min_overlap ? lo : min_overlap;
+    const float pairs = 1.25f * coverage, shifts = mo < max_len ? (float)(4 * (max_len - mo) + 2) : 2.0f;
+    // ns per pair on a full chip, by the words of a bit plane (registers of the scan)
+    const float pair = max_len <= 160 ? 0.03f + 0.00165f * shifts : max_len <= 192 ? 0.1f + 0.00175f * shifts
+                                                                                : 0.25f + 0.0019f * shifts;
+    const float column = 0.1f + 0.0011f * (float)max_len;
+    const float scan = pairs * (mirror ? 0.07f + 0.58f * pair : pair);
+    const float tc = 4.2f + pairs * (mirror ? 0.68f * column : column);
+    // us: the longest pair, the chain, and the anchors
+    const float n = 1e-3f * (float)anchors;
+    return !(fixed_us + 0.115f * shifts + n * scan < 12.5f + n * tc);
 }
 
 // 16 bases of a packed word -> 16 e4m3 bytes by their high bits, first base in

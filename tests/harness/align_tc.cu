@@ -170,3 +170,7 @@ extern "C" int hd_tc(const uint32_t* a, int La, const uint32_t* rows, int pitch,
     }
     return hits;
 }
+
+extern "C" int hd_tc_faster(int max_len, int min_overlap, float ratio, float coverage, unsigned anchors, int mirror) {
+    return tc_faster(max_len, min_overlap, ratio, coverage, anchors, mirror != 0, 0.0f);
+}

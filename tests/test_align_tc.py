@@ -158,6 +158,21 @@ def test_counts_of_an_overflowing_list(lib, seed):
     assert np.array_equal(out[0], out[1])
 
 
+@pytest.mark.parametrize("L,coverage,ratio,anchors,mirror,tensor", [
+    (36, 40, 0.3, 200_000, 0, 0), (50, 20, 0.3, 200_000, 0, 0), (50, 40, 0.3, 200_000, 0, 0),
+    (50, 30, 0.3, 200_000, 1, 0), (60, 20, 0.3, 200_000, 0, 0), (85, 10, 0.3, 200_000, 0, 0),
+    (85, 20, 0.3, 200_000, 0, 1), (100, 5, 0.3, 200_000, 0, 0), (100, 20, 0.3, 200_000, 0, 1),
+    (150, 5, 0.3, 200_000, 0, 0), (150, 10, 0.3, 200_000, 0, 1), (150, 30, 0.3, 200_000, 1, 1),
+    (100, 30, 0.8, 200_000, 0, 0), (150, 30, 0.9, 200_000, 0, 0), (150, 30, 0.6, 200_000, 0, 1),
+    (250, 5, 0.3, 200_000, 0, 1), (250, 30, 0.8, 200_000, 0, 1),
+    (50, 30, 0.3, 1000, 0, 0), (50, 5, 0.3, 4000, 0, 0), (70, 5, 0.3, 1000, 0, 1), (100, 5, 0.3, 128, 0, 1),
+    (150, 30, 0.3, 128, 0, 1)])
+def test_route_of_a_call(lib, L, coverage, ratio, anchors, mirror, tensor):
+    """The rule between the thread scan and the tensor cores at sizes where one
+    of them was measured to be 15 % or more ahead."""
+    assert lib.hd_tc_faster(L, 30, ctypes.c_float(ratio), ctypes.c_float(coverage), anchors, mirror) == tensor
+
+
 def test_random_pairs_rarely_stay_possible(lib):
     """The one-bit sums rule out nearly every shift of unrelated reads: that
     is what makes the exact counts few."""
