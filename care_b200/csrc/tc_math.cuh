@@ -99,9 +99,9 @@ inline uint32_t tc_splits(uint32_t anchors, uint32_t resident) {
 // tensor cores: 36 bases 5x 0.16, 0.91; 50 bases 20x 0.89, 1.33; 60 bases 40x
 // 2.20, 2.17; 100 bases 5x 0.70, 1.18, 10x 1.31, 1.40, 20x 2.54, 1.95; 150
 // bases 5x 1.02, 1.26, 10x 1.95, 1.55; 150 bases 30x with a minimum overlap of
-// 135 1.18, 2.09, of 90 3.29, 2.40; 250 bases 5x 2.47, 1.91; 1,000 anchors of
-// 50 bases 5x 0.018, 0.022, of 70 bases 0.029, 0.022. fixed_us: what the scan's
-// route adds to a call.
+// 135 1.18, 2.09, of 90 3.29, 2.40; 250 bases 5x 2.47, 1.91, 30x with a minimum
+// overlap of 225 4.33, 2.88; 1,000 anchors of 50 bases 5x 0.018, 0.022, of 70
+// bases 0.029, 0.022. fixed_us: what the scan's route adds to a call.
 inline bool tc_faster(int max_len, int min_overlap, float min_overlap_ratio, float coverage, uint32_t anchors,
                       bool mirror, float fixed_us) {
     const int lo = (int)((float)max_len * min_overlap_ratio), mo = lo > min_overlap ? lo : min_overlap;
@@ -109,7 +109,7 @@ inline bool tc_faster(int max_len, int min_overlap, float min_overlap_ratio, flo
     // ns per pair on a full chip, by the words of a bit plane (registers of the scan)
     const float pair = max_len <= 160 ? 0.03f + 0.00165f * shifts : max_len <= 192 ? 0.1f + 0.00175f * shifts
                                                                                 : 0.25f + 0.0019f * shifts;
-    const float column = 0.1f + 0.0011f * (float)max_len;
+    const float column = 0.12f + 0.0004f * (float)max_len + 0.085f * (float)((int)(0.5f * shifts + 127.0f) / 128 - 1);
     const float scan = pairs * (mirror ? 0.07f + 0.58f * pair : pair);
     const float tc = 4.2f + pairs * (mirror ? 0.68f * column : column);
     // us: the longest pair, the chain, and the anchors

@@ -164,7 +164,7 @@ def test_counts_of_an_overflowing_list(lib, seed):
     (85, 20, 0.3, 200_000, 0, 1), (100, 5, 0.3, 200_000, 0, 0), (100, 20, 0.3, 200_000, 0, 1),
     (150, 5, 0.3, 200_000, 0, 0), (150, 10, 0.3, 200_000, 0, 1), (150, 30, 0.3, 200_000, 1, 1),
     (100, 30, 0.8, 200_000, 0, 0), (150, 30, 0.9, 200_000, 0, 0), (150, 30, 0.6, 200_000, 0, 1),
-    (250, 5, 0.3, 200_000, 0, 1), (250, 30, 0.8, 200_000, 0, 1),
+    (250, 5, 0.3, 200_000, 0, 1), (250, 30, 0.8, 200_000, 0, 1), (250, 30, 0.9, 200_000, 0, 1),
     (50, 30, 0.3, 1000, 0, 0), (50, 5, 0.3, 4000, 0, 0), (70, 5, 0.3, 1000, 0, 1), (100, 5, 0.3, 128, 0, 1),
     (150, 30, 0.3, 128, 0, 1)])
 def test_route_of_a_call(lib, L, coverage, ratio, anchors, mirror, tensor):
