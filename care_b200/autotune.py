@@ -5,16 +5,22 @@ The knobs change how a batch is laid onto the GPU, never what it computes:
 - msa_order   anchors in longest-processing-time order (most candidates first)
 - msa_queue   persistent MSA CTAs pulling anchors from a device work queue
 - msa_warps   warps per anchor in the MSA stage (4 or 8)
-- align_block threads per CTA of the alignment stage (128 or 256)
-- pair_order  alignment pairs packed by candidate length within each anchor
 - graph       each batch's launches replayed as one CUDA graph
-- pair_mirror (a, c) and (c, a) of equal-length anchors of a batch share one scan
+- pair_mirror pairs (a, c) and (c, a) of a batch's anchors share one scan: of any
+  two lengths on the tensor cores, of equal lengths in the thread scan
 - cand_set_log2  capacity of the main candidate pass's de-duplication set
   (occupancy against anchors redone by the full-set pass)
-- align_warp  a warp per alignment work item (lanes take shifts) instead of
-  a thread per work item
-- align_classes  pairs partitioned by the plane width of their longer read,
-  one alignment launch per width
+- align_warp  the scan with a warp per alignment work item (lanes take shifts)
+  in place of the tensor cores
+- align_classes  the scan with pairs partitioned by the plane width of their
+  longer read, one launch per width, in place of the tensor cores (without
+  pair_mirror)
+
+and, where the mapping at hand runs the thread scan (they do nothing on the
+tensor cores):
+
+- align_block threads per CTA of the scan (128 or 256)
+- pair_order  alignment pairs packed by candidate length within each anchor
 
 Coordinate descent from the default: each knob in turn takes the value with
 the lowest device time (CUDA events of the pipeline, mean of timed passes
@@ -45,14 +51,13 @@ KNOBS = {
     "msa_order": [0, 1],
     "msa_queue": [0, 1],
     "msa_warps": [4, 8],
-    "align_block": [128, 256],
-    "pair_order": [0, 1],
     "graph": [0, 1],
     "pair_mirror": [0, 1],
     "cand_set_log2": [9, 10, 11],
     "align_warp": [0, 1],
     "align_classes": [0, 1],
 }
+SCAN_KNOBS = {"align_block": [128, 256], "pair_order": [0, 1]}
 DEFAULT = {"msa_order": 0, "msa_queue": 0, "msa_warps": 4, "align_block": 128, "pair_order": 0, "graph": 0,
            "pair_mirror": 0, "cand_set_log2": 10, "align_warp": 0, "align_classes": 0}
 
@@ -95,6 +100,17 @@ def measure(c: Corrector, tuning: dict, n: int, steps: int = 3) -> float:
     return float(np.mean(ms))
 
 
+def thread_scan(c: Corrector, tuning: dict, n: int) -> bool:
+    """Whether a form of the thread scan runs this mapping's alignment: only
+    there does pair_order launch a kernel of its own."""
+    launches = []
+    for v in (0, 1):
+        c.tuning = dict(tuning, pair_order=v)
+        c.correct_range_device(0, n)
+        launches.append(c.last_stats()["launches"])
+    return launches[0] != launches[1]
+
+
 def tune(c: Corrector, n: int, sweeps: int = 2, steps: int = 3, log=print) -> tuple[dict, dict]:
     c.tuning = DEFAULT
     ref = _fingerprint(c.correct_range(0, n))
@@ -113,7 +129,8 @@ def tune(c: Corrector, n: int, sweeps: int = 2, steps: int = 3, log=print) -> tu
     best = dict(DEFAULT)
     best_ms = timed(best)
     for _ in range(sweeps):
-        for k, values in KNOBS.items():
+        knobs = dict(KNOBS, **SCAN_KNOBS) if thread_scan(c, best, n) else KNOBS
+        for k, values in knobs.items():
             for v in values:
                 if v == best[k]:
                     continue
