@@ -915,7 +915,7 @@ int run_batch(care_b200_ctx* ctx, uint32_t first, uint32_t count, bool timed) {
     }
     const int warps = tu.msa_warps == 8 ? 8 : 4;
     const int nw = (ctx->max_len + 31) / 32;           // bit-plane width: 32-base words of the longest read
-    // length classes of the alignment (not with mirror pairs, whose work list pairs equal lengths)
+    // length classes of the scan (not with mirror pairs, whose work list has no classes)
     const bool classes = tu.align_classes != 0 && tu.pair_mirror == 0;
     if (classes) CK(ctx->d_cls.ensure(64), "alloc");
     // the tensor-core alignment, except for the statistics form, the mappings

@@ -3,7 +3,8 @@
 //   k_candidates : minhash signature + table lookup + de-duplication
 //                  (one CTA per anchor)
 //   k_align      : shifted Hamming distance, both strands, orientation,
-//                  pair flag (one thread per (anchor, candidate) pair)
+//                  pair flag (one thread per (anchor, candidate) pair); most
+//                  calls take k_align_tc (align_tc.cuh) in its place
 //   k_msa        : alignment filters, MSA build/refine, consensus
 //                  correction of anchor and candidates (one CTA per anchor)
 #pragma once
@@ -22,8 +23,9 @@ __constant__ float c_qweight[256];    // QualityScoreConversion table (qualitysc
 //                                     include/ordinaryminhasher.hpp:135-221,437-449
 //   determineCandidateReadIds         include/corrector.hpp:571-650
 // The table-major concatenation is followed by sort+unique in the reference;
-// here a shared-memory hash set removes duplicates and a bitonic sort orders
-// the (few) unique ids: same set, same ascending order.
+// here a shared-memory hash set removes duplicates, and the unique ids are
+// placed by counting the smaller ones (up to an id per thread) or by a bitonic
+// sort: same set, same ascending order.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 

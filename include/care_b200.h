@@ -208,9 +208,12 @@ int care_b200_last_timing(const care_b200_ctx* ctx, float* total_ms, float* stag
 
 /* Counters of the last correction call: stats[0] anchors, stats[1]
  * (anchor, candidate) pairs aligned, stats[2] candidate corrections,
- * stats[3] un-pruned 32-bit word compares of the alignment scans run (both
- * orientations, every scanned shift; a mirrored pair's shared scans count
- * once: the alignment stage's roofline work),
+ * stats[3] un-pruned 32-bit word compares of the alignment scans, run or
+ * answered by the tensor cores (both orientations, every scanned shift: the
+ * alignment stage's roofline work). Pairs that pair_mirror answers together
+ * count once, by the scan of their leading read: pairs of equal lengths in the
+ * scan and the statistics form, of any two lengths on the tensor cores, which
+ * is then the smaller count for reads of mixed lengths,
  * stats[4] bases of the MSAs' rows (anchor and candidates, every
  * build including refinement rebuilds: the MSA stage's compute work),
  * stats[5] device batches the range was split into, stats[6] kernels of
@@ -382,25 +385,34 @@ int care_b200_mlp_forward(care_b200_mlp* m, const float* x, uint64_t n, float* l
  *
  * How the batch's work is mapped onto the GPU; the results do not depend on
  * it (every variant is byte-identical). care_b200.autotune measures the
- * variants on a sample of a workload and commits the fastest per workload. */
+ * variants on a sample of a workload and commits the fastest per workload.
+ *
+ * The alignment runs on the tensor cores, or as a scan of the shifts with a
+ * thread per pair. The scan takes options the tensor-core bound does not cover
+ * (max_error_rate above 0.30, min_overlap below 1, a ratio outside [0, 1]), the
+ * statistics form (care_b200_count_word_compares), align_warp and
+ * align_classes, and calls with little work per pair or anchor (short reads, a
+ * minimum overlap near the read's length, low coverage). */
 typedef struct care_b200_tuning {
     int msa_order;     /* 1: anchors in longest-processing-time order (most candidates first) */
     int msa_queue;     /* 1: persistent MSA CTAs pulling anchors from a device work queue */
     int msa_warps;     /* warps per anchor in the MSA stage: 4 or 8 */
-    int align_block;   /* threads per CTA of the alignment stage: 128 or 256 */
-    int pair_order;    /* 1: alignment pairs packed by candidate length within each anchor */
+    int align_block;   /* threads per CTA of the scan: 128 or 256 (no effect on the tensor cores) */
+    int pair_order;    /* 1: the scan's pairs packed by candidate length within each anchor
+                          (no effect on the tensor cores) */
     int graph;         /* 1: each batch's launches replayed as one CUDA graph */
-    int pair_mirror;   /* 1: pairs (a, c) and (c, a) of equal-length anchors of one batch share
-                          their scans (one scan answers both forward alignments) */
+    int pair_mirror;   /* 1: pairs (a, c) and (c, a) whose reads are both anchors of the batch
+                          share their work: of any two lengths on the tensor cores, of equal
+                          lengths in the scan (one scan answers both forward alignments) */
     int cand_set_log2; /* 6..14: de-duplication set of the main candidate pass, 2^x entries;
                           anchors with more than 2^(x-1) unique candidates take a second pass
                           with a set for every retrieved id (default 10) */
-    int align_warp;    /* 1: a warp per alignment work item, its lanes taking the shifts of
-                          each group of 32 (the scan's first minimal shift found by warp
-                          reductions); 0: a thread per work item */
-    int align_classes; /* 1: the batch's pairs partitioned by the plane width their longer read
-                          needs (4/5/6/8 words of 32 bases), one alignment launch per class
-                          (no effect with pair_mirror) */
+    int align_warp;    /* 1: the scan, with a warp per alignment work item, its lanes taking the
+                          shifts of each group of 32 (the first minimal shift found by warp
+                          reductions) */
+    int align_classes; /* 1: the scan, with the batch's pairs partitioned by the plane width
+                          their longer read needs (4/5/6/8 words of 32 bases), one launch per
+                          class (no effect with pair_mirror) */
 } care_b200_tuning;
 
 int care_b200_default_tuning(care_b200_tuning* t);

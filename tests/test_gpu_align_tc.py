@@ -31,6 +31,8 @@ def _reads(seed, n, lo, hi, genome, rate=0.01):
 
 def _run(seqs, lengths, count_words, ranges, tuning=None, **opts):
     out = []
+    # mirrored pairs count once: on the tensor cores those of any two lengths, in the statistics form of equal lengths
+    same_count = not (tuning or {}).get("pair_mirror") or lengths.min() == lengths.max()
     with care_b200.Corrector(care_b200.default_options(**opts)) as c:
         c.upload_reads(care_b200.encode_reads(seqs, lengths), lengths)
         c.build_tables()
@@ -44,7 +46,8 @@ def _run(seqs, lengths, count_words, ranges, tuning=None, **opts):
                 assert (st["word_compares_run"] > 0) == count_words
             o = np.lexsort((r.cand_anchor_ids, r.cand_read_ids))
             out.append([r.status, r.num_edits, r.sequences, r.cand_read_ids[o], r.cand_anchor_ids[o], r.cand_shifts[o],
-                        r.cand_use_edits[o], r.cand_sequences[o], np.array([st["pairs"], 0 if (tuning or {}).get("pair_mirror") else st["word_compares"]])])
+                        r.cand_use_edits[o], r.cand_sequences[o],
+                        np.array([st["pairs"], st["word_compares"] if same_count else 0])])
     return out
 
 
