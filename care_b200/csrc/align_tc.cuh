@@ -28,13 +28,13 @@
 // would write them.
 //
 // Bound: instruction issue and barriers (57 % issue active and 13K warp
-// instructions per anchor of 47 candidates, with mirrors 68 % and 8.6K; the
+// instructions per anchor of 47 candidates, with mirrors 69 % and 8.8K; the
 // products take a tenth of the tensor pipe, 46 cycles per 128 x 64 x 32 step,
 // the same as with a stored Toeplitz matrix). Measured against the thread scan
 // (k_align) and its pair mirroring: 1M 150 bp paired-end reads at 30x 14.3 ms
 // (18.8), 1.3M at 50x 24.3 ms (36.3), 400k reads of 50-250 bases 11.8 ms with
 // mirrors, 18.0 ms without (34.1), 300k 100 bp reads 3.1 and 4.1 ms (5.6), 128
-// anchors 28 us (58).
+// anchors 26 us (58). Where the scan is faster: tc_faster.
 #pragma once
 #include "kernels.cuh"
 #include "tc05.cuh"
@@ -615,7 +615,7 @@ k_align_tc(DevOptions o, DevReads r, uint32_t first, uint32_t count, const uint3
     }
 done:
     if (bad) {
-        if (tid == 0) atomicOr(status, kStatusTensorWait);
+        if (tid == 0) atomicOr(status, kStatusTensorWait | kStatusIncomplete);
         tc05::mbar_wait(&s_bar, phase ^ 1u);            // the product in flight ends before its memory is released
     }
     if (work_count) {

@@ -229,7 +229,7 @@ __device__ __forceinline__ void candidates_of(
         const unsigned long long at = s_base;
         if (tid == 0) { seg_off[ai] = (uint32_t)at; seg_cnt[ai] = U; }
         if (at + U > arena_cap) {
-            if (tid == 0) atomicOr(status, kStatusCandOverflow);
+            if (tid == 0) atomicOr(status, kStatusCandOverflow | kStatusIncomplete);
             return;
         }
         if ((uint32_t)tid < U) {
@@ -281,7 +281,7 @@ __device__ __forceinline__ void candidates_of(
     const unsigned long long base = s_base;
     if (tid == 0) { seg_off[ai] = (uint32_t)base; seg_cnt[ai] = U; }
     if (base + U > arena_cap) {
-        if (tid == 0) atomicOr(status, kStatusCandOverflow);
+        if (tid == 0) atomicOr(status, kStatusCandOverflow | kStatusIncomplete);
         return;
     }
     for (uint32_t i = tid; i < U; i += BLOCK) { cand_ids[base + i] = list[i]; cand_anchor[base + i] = ai; }
@@ -779,7 +779,7 @@ k_align_warp(DevOptions o, DevReads r, uint32_t first, const uint32_t* __restric
 // Bound: instruction issue. Measured against sums of every column with the
 // rows staged whole: 1M 150 bp paired-end reads at 30x 13.0 ms (20.7), 400k
 // reads of 50-250 bases 8.8 ms (18.2), 1.3M reads at 50x 22.4 ms (38.4), 128
-// anchors 0.17 ms (0.45).
+// anchors 66 us (168).
 // ---------------------------------------------------------------------------
 struct MsaOut {
     uint8_t* status;
@@ -1672,7 +1672,7 @@ msa_anchor(const DevOptions& o, const DevReads& r, uint32_t first, uint32_t ai, 
 // anchors enough to fill them, the register limit of ten is taken (48
 // registers, a few spills): 12.6 -> 12.0 ms per 1M 150 bp reads. Reads of
 // 50-250 bases, which shared memory holds to eight, lose by it (8.5 -> 8.9 ms
-// per 400k), and so do 128 anchors, one per SM (156 -> 217 us).
+// per 400k), and so do 128 anchors, one per SM (66 -> 88 us).
 constexpr int kMsaManyCtas = 10;
 inline bool msa_many_ctas(size_t dynamic_smem, uint32_t anchors, int sms) {
     return (dynamic_smem + 8192) * kMsaManyCtas <= 228 * 1024 && anchors >= (uint32_t)(16 * sms);

@@ -15,7 +15,7 @@ SRC = os.path.join(ROOT, "tests", "harness", "tensor_wait.cu")
 OUT = os.path.join(ROOT, "tests", "_build", "libtensor_wait.so")
 CSRC = os.path.join(ROOT, "care_b200", "csrc")
 DEPS = [SRC] + [os.path.join(CSRC, f) for f in ("device.cuh", "tc_math.cuh", "tc05.cuh", "kernels.cuh", "align_tc.cuh")]
-TENSOR_WAIT = 16                                     # kStatusTensorWait
+TENSOR_WAIT = 16 | 32                                # kStatusTensorWait | kStatusIncomplete
 LIMIT = 1 << 22                                      # kTcWaitLimit
 
 
