@@ -69,7 +69,7 @@ MLP_FILE = os.path.join(ROOT, "care_b200", "data", "mlp_pe30x.bin")
 # k_msa DRAM bytes per anchor: dram__bytes_read.sum + dram__bytes_write.sum of
 # one ncu capture of 100,000 anchors of this workload model (69.45 MB read +
 # 4.59 MB written)
-MSA_DRAM_BYTES_PER_ANCHOR = 740.0
+MSA_DRAM_BYTES_PER_ANCHOR = 733.0
 CARE_CPU = os.path.join(ROOT, "oracle", "_ref", "care-cpu")
 L2_BYTES = 126 * 1024 * 1024
 
